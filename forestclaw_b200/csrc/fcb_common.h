@@ -41,6 +41,7 @@ enum { MLP_BLOB_F_B1 = 0, MLP_BLOB_F_B2 = 64, MLP_BLOB_F_W3 = 128, MLP_BLOB_F_B3
 struct LevelGroup {
     int nlev;
     int start[34];
+    int seeded;         // exact Euler: Newton starts from the p*-seed network
 };
 
 struct StepParams {

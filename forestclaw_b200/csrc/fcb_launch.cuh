@@ -15,11 +15,20 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <utility>
+#include "fcb_common.h"
 
 namespace fcb {
 
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Parameter block of relative patch b of a launch over lg.nlev levels.
+__device__ __forceinline__ int group_slot(const LevelGroup& lg, int b)
+{
+    int k = 0;
+    for (int i = 1; i < lg.nlev; i++) k += (b >= lg.start[i]) ? 1 : 0;
+    return lg.nlev - 1 - k;
+}
 
 // Host flag of the calling thread: launches through launch_k carry the
 // programmatic-serialization attribute while it is set (ProgrammaticScope).

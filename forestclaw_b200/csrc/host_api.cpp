@@ -30,23 +30,21 @@ static double wall_ms()
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-// A specialised kernel (spec = its limiter) applies to the second-order method with
-// second-order transverse terms, that limiter on every one of 3 waves of 3 fields, no
-// capacity, no aux and no cubed sphere.
+// A variant with the method fixed at compile time (spec = its limiter) applies to the
+// second-order method with second-order transverse terms, that limiter on every one of the
+// three waves and no capacity.
 static bool spec_applies(const Step2Variant& v, const fc2d_b200_options_t& o)
 {
     if (v.spec == 0) return true;
-    if (o.order[0] != 2 || o.order[1] != 2 || o.mcapa != 0 || o.maux != 0 || o.meqn != 3 || o.mwaves != 3 ||
-        o.app == FC2D_B200_APP_SPHERE)
-        return false;
+    if (o.order[0] != 2 || o.order[1] != 2 || o.mcapa != 0) return false;
     for (int w = 0; w < 3; w++)
         if (o.mthlim[w] != v.spec) return false;
     return true;
 }
 
 // Patch-to-CTA variants of the fused update compiled for one solver shape (first: default).
-// Where a specialised kernel applies, only its variants are offered, so that every
-// variant the autotuner may pick gives the same results.
+// Where variants with a compile-time method apply, only they are offered: they do the
+// same arithmetic with fewer instructions.
 static std::vector<const Step2Variant*> step2_variants(const fc2d_b200_options_t& o, int rp)
 {
     using Table = const Step2Variant* (*)(int*);
@@ -591,6 +589,7 @@ static int flush_updates(fc2d_b200_solver* s)
     if (s->timing) { e0 = next_event(s); e1 = next_event(s); CK(cudaEventRecord(e0, s->st)); }
     LevelGroup lg{};
     lg.nlev = g.lev_hi - g.lev_lo + 1;
+    lg.seeded = s->use_mlp;
     for (int i = 0; i < lg.nlev; i++)
         lg.start[i] = (s->part ? s->part->plan.own_lo[g.lev_lo + i] : s->forest.lev_off[g.lev_lo + i]) - g.p0;
     cudaError_t e = s->vars[g.var]->fn(s->q, s->qlast, s->aux, s->regs, s->desc, g.p0, g.np, s->params_dev + g.slot,
@@ -2599,6 +2598,7 @@ extern "C" int fc2d_b200_set_pstar_seed(fc2d_b200_solver_t* s, const fc2d_b200_m
 {
     DeviceScope dev_scope_(s);
     if (!s) return fail(FC2D_B200_EINVAL, "null solver");
+    if (s->use_mlp != (m != nullptr)) invalidate_graph(s);   // seeded and unseeded updates are different kernels
     if (!m) { s->use_mlp = false; return 0; }
     if (s->o.rp != FC2D_B200_RP_EULER_EXACT) return fail(FC2D_B200_EINVAL, "the p* seed applies to the Euler solver");
     if (!s->mlp_blob) CK(cudaMalloc(&s->mlp_blob, MLP_BLOB_BYTES));
@@ -2763,6 +2763,8 @@ extern "C" int fc2d_b200_autotune(fc2d_b200_solver_t* s, int reps, int* best_out
     StepParams sp = make_params(s, f.maxlevel_present, s->t_curr, 0.0);
     sp.store_flux = 0; sp.accumulate_waves = 0; sp.save_last = 0; sp.newton_hist = nullptr;
     CK(cudaMemcpyAsync(s->tune_params, &sp, sizeof(StepParams), cudaMemcpyHostToDevice, s->st));
+    LevelGroup one{1, {0}};                       // one level per launch
+    one.seeded = s->use_mlp;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
@@ -2770,7 +2772,7 @@ extern "C" int fc2d_b200_autotune(fc2d_b200_solver_t* s, int reps, int* best_out
         for (int l = 0; l <= 32; l++) {
             const int p0 = f.lev_off[l], np = f.lev_off[l + 1] - p0;
             if (np <= 0) continue;
-            cudaError_t e = v->fn(s->q, s->qlast, s->aux, s->regs, s->desc, p0, np, s->tune_params, LevelGroup{1, {0}}, s->cfl_dev, s->st);
+            cudaError_t e = v->fn(s->q, s->qlast, s->aux, s->regs, s->desc, p0, np, s->tune_params, one, s->cfl_dev, s->st);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
@@ -2796,10 +2798,10 @@ extern "C" int fc2d_b200_autotune(fc2d_b200_solver_t* s, int reps, int* best_out
     // on it alone (by 5 %: the forest changes between regrids, and a small level's
     // launch is a few microseconds); each level's timing covers at least ~0.3 ms
     auto time_level = [&](const Step2Variant* x, int p0, int np, int n, double& per) -> cudaError_t {
-        cudaError_t e = x->fn(s->q, s->qlast, s->aux, s->regs, s->desc, p0, np, s->tune_params, LevelGroup{1, {0}}, s->cfl_dev, s->st);
+        cudaError_t e = x->fn(s->q, s->qlast, s->aux, s->regs, s->desc, p0, np, s->tune_params, one, s->cfl_dev, s->st);
         if (e == cudaSuccess) e = cudaEventRecord(e0, s->st);
         for (int r = 0; r < n && e == cudaSuccess; r++)
-            e = x->fn(s->q, s->qlast, s->aux, s->regs, s->desc, p0, np, s->tune_params, LevelGroup{1, {0}}, s->cfl_dev, s->st);
+            e = x->fn(s->q, s->qlast, s->aux, s->regs, s->desc, p0, np, s->tune_params, one, s->cfl_dev, s->st);
         if (e == cudaSuccess) e = cudaEventRecord(e1, s->st);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         float ms = 0.0f;

@@ -13,14 +13,14 @@
 //   the conservative q update over i,j = 1-mbc..mx+mbc-1 (clawpack46_step2_wrap.f:107-125)
 //   and the warp-shuffle CFL maximum.
 //
+// It serves the scalar advection apps and application solvers; the flux-form systems
+// (shallow water, Euler) have their own kernel, k_wave.cuh.
+//
 // TW is the arithmetic type of the waves, speeds, limiter, second-order
 // correction and transverse splitting.  TW = double is the FP64 path (built
 // without FMA contraction: bitwise equal to the FP64 CPU path).  TW = float is
-// the FP32-wave path: the flux arrays fm/fp/gm/gp, the q update, the time-sync
-// registers and the CFL reduction stay FP64, and the Godunov split is taken as
-// an FP64 remainder, amdq = [f(q_i) - f(q_{i-1})](FP64) - apdq, so that
-// amdq + apdq telescopes to FP64 round-off and mass stays conserved to
-// FP64 accuracy although the waves are FP32.
+// the FP32-wave path: the Godunov split, the flux arrays fm/fp/gm/gp, the q update,
+// the time-sync registers and the CFL reduction stay FP64.
 //
 // Index conventions: padded 0-based cell (ic, jc), ic = i + mbc - 1 for the
 // Fortran index i.  Interface ic sits between cells ic-1 and ic.
@@ -30,7 +30,6 @@
 #include "fcb_common.h"
 #include "fcb_launch.cuh"
 #include "riemann.cuh"
-#include "k_mlp.cuh"
 
 namespace fcb {
 
@@ -41,11 +40,6 @@ enum { APP_NONE = 0, APP_SWIRL = 1, APP_RADIALDAM = 2, APP_TSUNAMI = 3, APP_SHOC
 // include/fc2d_b200_user.cuh, and AUX_BOTH = true to receive in rpt2 the aux of
 // both cells beside the interface, cudaclaw's layout (cudaclaw_flux2.cu:682-694):
 // aux1/aux2/aux3[imp * maux + m], imp = 0 for the left cell, 1 for the right.
-// Solvers whose field 0 is a water depth declare DEPTH = true: a negative depth is
-// reported through the status word.
-template <class RP, class = void> struct RPDepth { static constexpr bool value = false; };
-template <class RP> struct RPDepth<RP, std::void_t<decltype(RP::DEPTH)>> { static constexpr bool value = RP::DEPTH; };
-
 template <class RP, class = void>
 struct RPHooks { static constexpr bool B4 = false, SRC = false, AUX_BOTH = false; };
 template <class RP>
@@ -75,9 +69,7 @@ struct Step2Geom {
     // per-interface transverse terms: A1, A2 (from amdq), B1, B2 (from apdq)
     static constexpr int TSZ = 4 * MEQN;
     static constexpr int AUXS = MAUX > 0 ? MAUX : 0;
-    static constexpr bool USE_FLX = F32 && RP::CONS_FLUX;   // per-cell FP64 fluxes (remainder / Godunov split)
-    static constexpr size_t DOUBLES = (size_t)MEQN * NXY * 5 + (size_t)AUXS * NXY +
-                                      (USE_FLX ? (size_t)MEQN * NXY : 0) + 64;
+    static constexpr size_t DOUBLES = (size_t)MEQN * NXY * 5 + (size_t)AUXS * NXY + 64;
     static constexpr size_t TWS = (size_t)WSZ * NI + (size_t)TSZ * NI + (F32 ? (size_t)MEQN * NXY : 0);
     static constexpr size_t SMEM_BYTES = DOUBLES * 8 + TWS * sizeof(TW) + NI;
     // conservation registers (fclaw2d_clawpatch_conservation.h:56-77), per patch
@@ -89,41 +81,16 @@ struct Step2Geom {
                          NREG = R_EF3 + 2 * MX * MEQN;
 };
 
-// Shallow-water flux function used by the time-sync flux store
-// (applications/clawpack/shallow/2d/radialdam/rpn2cons_update.f).
-template <typename T>
-__device__ __forceinline__ void rpn2_cons_sw(int idir, const T* q, T grav, T* flux)
-{
-    const int mu = (idir == 0) ? 1 : 2, mv = (idir == 0) ? 2 : 1;
-    T hun = q[mu], hut = q[mv], h = q[0];
-    T un = hun / h;
-    flux[0] = hun;
-    flux[mu] = (hun * hun) / h + T(0.5) * grav * (h * h);
-    flux[mv] = un * hut;
-}
-
-// Correctly rounded, uncontracted multiply / add.  The FP32-wave unit is built with
-// FMA contraction; the second-order correction must not be contracted, or the
-// exactly opposite terms of the waves at a reflecting wall leave the rounding
-// error of one product as a flux through the wall.
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-
 // The update of patch p by the whole CTA (one call per patch; the CTA may do
-// several patches in turn).  nhist: the CTA's shared Newton-iteration counters.
+// several patches in turn).
 template <class RP, int MX, int MY, int MBC, bool FWAVE, int NT, typename TW>
 __device__ __forceinline__ void
 step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __restrict__ aux,
             double* __restrict__ regs, const PatchDesc* __restrict__ desc, const int p,
-            const StepParams& sp, unsigned long long* __restrict__ cfl_bits, unsigned int* nhist)
+            const StepParams& sp, unsigned long long* __restrict__ cfl_bits)
 {
     using G = Step2Geom<RP, MX, MY, MBC, TW, NT>;
     constexpr bool F32 = G::F32, REG = G::REG;
-    static_assert(!RP::EXACT64 || G::REG, "exact solvers keep their FP64 fluctuations in registers");
     constexpr int NX = G::NX, NY = G::NY, NXY = G::NXY, MEQN = G::MEQN, MWAVES = G::MWAVES;
     constexpr int MAUX = G::MAUX, NEXTRA = G::NEXTRA, NI = G::NI, WSZ = G::WSZ;
     constexpr int MA = MAUX > 0 ? MAUX : 1;
@@ -144,15 +111,13 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     double* GMs = FPs + MEQN * NXY;
     double* GPs = GMs + MEQN * NXY;
     double* As = GPs + MEQN * NXY;                  // [MAUX][NY][NX]
-    double* FLX = As + G::AUXS * NXY;               // [MEQN][NY][NX] cell fluxes (FP32-wave path)
-    double* red = FLX + (G::USE_FLX ? MEQN * NXY : 0);   // 64 doubles for reductions
+    double* red = As + G::AUXS * NXY;               // 64 doubles for reductions
     TW* W = reinterpret_cast<TW*>(red + 64);        // [WSZ][NI]  (SoA)
     TW* Tt = W + (size_t)WSZ * NI;                  // [TSZ][NI]
     TW* Qf = Tt + (size_t)G::TSZ * NI;              // [MEQN][NY][NX] q in TW (FP32-wave path)
     unsigned char* tflag = reinterpret_cast<unsigned char*>(Qf + (F32 ? MEQN * NXY : 0));
 
     const int tid = threadIdx.x;
-    if (RP::EXACT64 && tid < 32) nhist[tid] = 0u;          // Newton iterations of this patch
     const PatchDesc pd = desc[p];
     const double dx = pd.dx, dy = pd.dy;
     const double dt = sp.inst_dt ? sp.dt * sp.inst_dt[pd.inst] : sp.dt;
@@ -167,7 +132,6 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     for (int k = tid; k < MEQN * NXY; k += NT) {
         double v = qg[k];
         if (!isfinite(v)) bad |= STATUS_NONFINITE;
-        if constexpr (RPDepth<RP>::value) { if (k < NXY && v < 0.0) bad |= STATUS_DEPTH; }
         Qs[k] = v;
         if (F32) Qf[k] = (TW)v;
         if (save) qlast[(size_t)p * MEQN * NXY + k] = v;
@@ -219,97 +183,18 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     };
     const TW gravw = (TW)sp.grav, drytolw = (TW)sp.dry_tolerance;
 
-    // ---- time-sync flux store (before the update), FP64 ----------------------
     double* rg = regs + (size_t)p * G::NREG;
-    if (MEQN >= 3 && sp.store_flux) {
-        // faces 0,1: j = 1..my, k = 0,1 ; faces 2,3: i = 1..mx, k = 0,1
-        for (int it = tid; it < 2 * 2 * MY + 2 * 2 * MX; it += NT) {
-            int face, j, k;
-            if (it < 4 * MY) { face = it / (2 * MY); int r = it % (2 * MY); j = r / 2; k = r % 2; }
-            else { int r2 = it - 4 * MY; face = 2 + r2 / (2 * MX); int r = r2 % (2 * MX); j = r / 2; k = r % 2; }
-            int ic, jc;
-            if (face == 0) { ic = MBC - k; jc = MBC + j; }
-            else if (face == 1) { ic = MX + MBC - 1 + k; jc = MBC + j; }
-            else if (face == 2) { ic = MBC + j; jc = MBC - k; }
-            else { ic = MBC + j; jc = MY + MBC - 1 + k; }
-            double qv[MEQN >= 3 ? MEQN : 3], fl[MEQN >= 3 ? MEQN : 3];
-            for (int m = 0; m < MEQN; m++) qv[m] = Qs[m * NXY + jc * NX + ic];
-            if constexpr (RP::EXACT64) { RP::cons_flux(face / 2, qv, sp.gamma, fl); }
-            else { rpn2_cons_sw<double>(face / 2, qv, sp.grav, fl); }
-            const int n = (face < 2) ? MY : MX;
-            const double el = (face < 2) ? dy : dx;
-            const int base = (face == 0) ? G::R_EF0 : (face == 1) ? G::R_EF1 : (face == 2) ? G::R_EF2 : G::R_EF3;
-            const bool zero = (sp.reg_reset >> ((pd.face_type >> (2 * face)) & 3)) & 1;
-            for (int m = 0; m < MEQN; m++) {
-                double* r = &rg[base + j + m * n + k * n * MEQN];
-                *r = (zero ? 0.0 : *r) + dt * el * fl[m];
-            }
-        }
-    }
-
     double cflmax = 0.0;
     TW cflw = TW(0);
 
-    // Reflecting walls of this patch (FP32-wave path).  Mirror symmetry makes the
-    // mass flux through a wall exactly zero -- first-order part, second-order
-    // correction and the transverse terms of the two rows (columns) beside it
-    // cancel -- but FP32 waves only reproduce that cancellation to FP32 rounding,
-    // which leaks about 1e-8 of the mass per step.  The FP32-wave path therefore
-    // takes the exact value, zero, for the mass component (m = 0) at these faces;
-    // the FP64 path keeps the reference's arithmetic.
-    const int wallf = (F32 && RP::CONS_FLUX) ? (pd.phys_mask & sp.wall_faces) : 0;
-
-    // g64: FP64 amdq, apdq of exact solvers (kept for the Godunov update)
-    struct State { TW wave[MWAVES][MEQN]; TW s[MWAVES]; TW am[MEQN]; TW ap[MEQN]; TW ex[NEXTRA];
-                   double g64[RP::EXACT64 ? 2 * MEQN : 1]; };
+    struct State { TW wave[MWAVES][MEQN]; TW s[MWAVES]; TW am[MEQN]; TW ap[MEQN]; TW ex[NEXTRA]; };
 
     // Normal solve of one interface (qL = cell cL, qR = cell cR).
-    auto normal_solve = [&](int ixy, int cL, int cR, int k, bool cfl_range, TW d1, TW d0, State& st, double seed) {
-        if constexpr (RP::EXACT64 && F32) {
-            float qL[MEQN], qR[MEQN], w32[MWAVES][MEQN], s32[MWAVES], ex32[NEXTRA];
-            double qL64[MEQN], qR64[MEQN], fL[MEQN], fR[MEQN], am64[MEQN], ap64[MEQN];
-            for (int m = 0; m < MEQN; m++) {
-                qL[m] = Qf[m * NXY + cL]; qR[m] = Qf[m * NXY + cR];
-                qL64[m] = Qs[m * NXY + cL]; qR64[m] = Qs[m * NXY + cR];
-                fL[m] = FLX[m * NXY + cL]; fR[m] = FLX[m * NXY + cR];
-            }
-            const EulerParams ep{sp.gamma, sp.newton_tol, seed};
-            const int r = RP::solve_mixed(ixy, qL, qR, qL64, qR64, fL, fR, ep, w32, s32, am64, ap64, ex32);
-            const int it = r & 0xff;
-            atomicAdd(&nhist[it < 31 ? it : 31], 1u);
-            if ((r & RP::NEWTON_FAILED) && sp.status) atomicOr(sp.status, (unsigned)STATUS_NEWTON);
-            for (int mw = 0; mw < MWAVES; mw++) {
-                st.s[mw] = (TW)s32[mw];
-                for (int m = 0; m < MEQN; m++) st.wave[mw][m] = (TW)w32[mw][m];
-            }
-            for (int m = 0; m < MEQN; m++) {
-                st.am[m] = (TW)am64[m]; st.ap[m] = (TW)ap64[m];
-                st.g64[m] = am64[m]; st.g64[MEQN + m] = ap64[m];
-            }
-            for (int e = 0; e < NEXTRA; e++) st.ex[e] = (TW)ex32[e];
-        } else if constexpr (RP::EXACT64) {
-            double qL64[MEQN], qR64[MEQN], w64[MWAVES][MEQN], s64[MWAVES], am64[MEQN], ap64[MEQN], ex64[NEXTRA];
-            for (int m = 0; m < MEQN; m++) { qL64[m] = Qs[m * NXY + cL]; qR64[m] = Qs[m * NXY + cR]; }
-            const EulerParams ep{sp.gamma, sp.newton_tol, seed};
-            const int r = RP::solve64(ixy, qL64, qR64, ep, w64, s64, am64, ap64, ex64);
-            const int it = r & 0xff;
-            atomicAdd(&nhist[it < 31 ? it : 31], 1u);
-            if ((r & RP::NEWTON_FAILED) && sp.status) atomicOr(sp.status, (unsigned)STATUS_NEWTON);
-            for (int mw = 0; mw < MWAVES; mw++) {
-                st.s[mw] = (TW)s64[mw];
-                for (int m = 0; m < MEQN; m++) st.wave[mw][m] = (TW)w64[mw][m];
-            }
-            for (int m = 0; m < MEQN; m++) {
-                st.am[m] = (TW)am64[m]; st.ap[m] = (TW)ap64[m];
-                st.g64[m] = am64[m]; st.g64[MEQN + m] = ap64[m];
-            }
-            for (int e = 0; e < NEXTRA; e++) st.ex[e] = (TW)ex64[e];
-        } else {
-            TW qL[MEQN], qR[MEQN], aL[MA], aR[MA];
-            for (int m = 0; m < MEQN; m++) { qL[m] = qload(m, cL); qR[m] = qload(m, cR); }
-            for (int a = 0; a < MAUX; a++) { aL[a] = (TW)As[a * NXY + cL]; aR[a] = (TW)As[a * NXY + cR]; }
-            RP::template rpn2<TW>(ixy, qL, qR, aL, aR, st.wave, st.s, st.am, st.ap, st.ex, gravw);
-        }
+    auto normal_solve = [&](int ixy, int cL, int cR, int k, bool cfl_range, TW d1, TW d0, State& st) {
+        TW qL[MEQN], qR[MEQN], aL[MA], aR[MA];
+        for (int m = 0; m < MEQN; m++) { qL[m] = qload(m, cL); qR[m] = qload(m, cR); }
+        for (int a = 0; a < MAUX; a++) { aL[a] = (TW)As[a * NXY + cL]; aR[a] = (TW)As[a * NXY + cR]; }
+        RP::template rpn2<TW>(ixy, qL, qR, aL, aR, st.wave, st.s, st.am, st.ap, st.ex, gravw);
         for (int mw = 0; mw < MWAVES; mw++)
             for (int m = 0; m < MEQN; m++) W[(G::W_WAVE + mw * MEQN + m) * NI + k] = st.wave[mw][m];
         if (!REG) {
@@ -344,25 +229,12 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
                                 double* faddm, double* faddp) {
         TW cq[MEQN];
         for (int m = 0; m < MEQN; m++) { cq[m] = TW(0); faddm[m] = 0.0; faddp[m] = 0.0; }
-        // wall_lo: ghost on the left (low face), wall_hi: ghost on the right (high face)
-        const bool wall_lo = wallf && pos == lim_lo && (wallf & (ixy == 1 ? 1 : 4));
-        const bool wall_hi = wallf && pos == lim_hi && (wallf & (ixy == 1 ? 2 : 8));
         if (god) {
-            if constexpr (RP::EXACT64) {
-                for (int m = 0; m < MEQN; m++) { faddp[m] = faddp[m] - st.g64[MEQN + m]; faddm[m] = faddm[m] + st.g64[m]; }
-            } else if constexpr (F32) {
-                double am64[MEQN], ap64[MEQN];
-                double qL[MEQN], qR[MEQN], aL[MA], aR[MA], fL[MEQN], fR[MEQN];
-                for (int m = 0; m < MEQN; m++) {
-                    qL[m] = Qs[m * NXY + cL]; qR[m] = Qs[m * NXY + cR];
-                    if (G::USE_FLX) { fL[m] = FLX[m * NXY + cL]; fR[m] = FLX[m * NXY + cR]; }
-                    else { fL[m] = 0.0; fR[m] = 0.0; }
-                }
-                for (int a = 0; a < MAUX; a++) { aL[a] = As[a * NXY + cL]; aR[a] = As[a * NXY + cR]; }
-                RP::godunov64(ixy, qL, qR, aL, aR, fL, fR, st.ap, am64, ap64, sp.grav);
-                // zero mass flux through a wall: the interior cell's fluctuation cancels its own flux
-                if (wall_lo) { ap64[0] = fR[0]; am64[0] = (fR[0] - fL[0]) - fR[0]; }
-                if (wall_hi) { am64[0] = 0.0 - fL[0]; ap64[0] = (fR[0] - fL[0]) + fL[0]; }
+            if constexpr (F32) {
+                double am64[MEQN], ap64[MEQN], qL[MEQN], qR[MEQN], aR[MA];
+                for (int m = 0; m < MEQN; m++) { qL[m] = Qs[m * NXY + cL]; qR[m] = Qs[m * NXY + cR]; }
+                for (int a = 0; a < MAUX; a++) aR[a] = As[a * NXY + cR];
+                RP::godunov64(ixy, qL, qR, aR, am64, ap64);
                 for (int m = 0; m < MEQN; m++) { faddp[m] = faddp[m] - ap64[m]; faddm[m] = faddm[m] + am64[m]; }
             } else {
                 for (int m = 0; m < MEQN; m++) { faddp[m] = faddp[m] - (double)st.ap[m]; faddm[m] = faddm[m] + (double)st.am[m]; }
@@ -404,7 +276,6 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
                             c = add_rn(c, mul_rn(mul_rn(sa, sub_rn(TW(1), mul_rn(sa, dave))), st.wave[mw][m]));
                         }
                     }
-                    if (m == 0 && (wall_lo || wall_hi)) c = TW(0);
                     cq[m] = c;
                     if (F32) {
                         const double h = 0.5 * (double)c;
@@ -481,59 +352,12 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
         }
     };
 
-    // cell fluxes for the FP64 remainder of the Godunov split
-    auto cell_fluxes = [&](int ixy) {
-        if constexpr (G::USE_FLX) {
-            for (int c = tid; c < NXY; c += NT) {
-                double qv[MEQN], fv[MEQN];
-                for (int m = 0; m < MEQN; m++) qv[m] = Qs[m * NXY + c];
-                RP::flux64(ixy, qv, RP::EXACT64 ? sp.gamma : sp.grav, fv);
-                for (int m = 0; m < MEQN; m++) FLX[m * NXY + c] = fv[m];
-            }
-        }
-    };
-
-    // p*-seed of the exact solver for interface k of sweep ixy (all lanes of the
-    // warp take part; k < 0 marks a lane without an interface)
-    auto mlp_seed = [&](int ixy, int k) -> double {
-        if constexpr (RP::EXACT64) {
-            int cL = 0, cR = 1;
-            if (k >= 0) {
-                if (ixy == 1) { const int jc = 1 + k / (NX - 1), ic = 1 + k % (NX - 1); cL = jc * NX + ic - 1; cR = cL + 1; }
-                else { const int jc = 1 + k / (NX - 2), ic = 1 + k % (NX - 2); cL = (jc - 1) * NX + ic; cR = cL + NX; }
-            }
-            double qL[MEQN], qR[MEQN];
-            for (int m = 0; m < MEQN; m++) { qL[m] = Qs[m * NXY + cL]; qR[m] = Qs[m * NXY + cR]; }
-            const typename RP::Prim P = RP::prim(ixy, qL, qR, sp.gamma);
-            float x[MLP_IN];
-            double pbase;
-            mlp_features(P.rl, P.ul, P.pl, P.rr, P.ur, P.pr, sp.gamma, x, pbase);
-            if (k < 0 || !(x[0] == x[0] && x[1] == x[1] && x[2] == x[2] && x[3] == x[3] && x[4] == x[4] && x[5] == x[5])) {
-                x[0] = 1.0f; x[1] = 0.0f; x[2] = 1.0f; x[3] = 1.0f; x[4] = 0.0f; x[5] = 1.0f;
-                k = -1;
-            }
-            const bool use = k >= 0 && mlp_gate(x);
-            // the network runs per warp (mma.sync over its 32 interfaces): skip warps
-            // without an interface past the gate (smooth flow, weak waves)
-            if (!__any_sync(0xffffffffu, use)) return 0.0;
-            const MlpView W(sp.mlp);
-            MlpFrag h1, h2;
-            mlp_warp_hidden<true>(W, x, h1, h2);
-            const float y = mlp_warp_output(W, h2);
-            if constexpr (F32) { return use ? pbase * (double)__expf(y) : 0.0; }
-            else { return use ? pbase * fcb_exp((double)y) : 0.0; }
-        } else {
-            (void)ixy; (void)k;
-            return 0.0;
-        }
-    };
-
     // x-sweep interface k -> row jc = 1 + k / (NX-1), interface ic = 1 + k % (NX-1)
-    auto x1 = [&](int k, State& st, double seed) {
+    auto x1 = [&](int k, State& st) {
         const int jc = 1 + k / (NX - 1), ic = 1 + k % (NX - 1);
         const bool cr = (ic >= MBC && ic <= MX + MBC);
         normal_solve(1, jc * NX + ic - 1, jc * NX + ic, k, cr, cr ? dtdx1d_x(ic, jc) : TW(0),
-                     cr ? dtdx1d_x(ic - 1, jc) : TW(0), st, seed);
+                     cr ? dtdx1d_x(ic - 1, jc) : TW(0), st);
     };
     auto x2 = [&](int k, State& st) {
         const int jc = 1 + k / (NX - 1), ic = 1 + k % (NX - 1);
@@ -554,11 +378,11 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
         }
     };
     // y-sweep interface k -> row interface jc = 1 + k / (NX-2), column ic = 1 + k % (NX-2)
-    auto y1 = [&](int k, State& st, double seed) {
+    auto y1 = [&](int k, State& st) {
         const int jc = 1 + k / (NX - 2), ic = 1 + k % (NX - 2);
         const bool cr = (jc >= MBC && jc <= MY + MBC);
         normal_solve(2, (jc - 1) * NX + ic, jc * NX + ic, k, cr, cr ? dtdy1d_y(ic, jc) : TW(0),
-                     cr ? dtdy1d_y(ic, jc - 1) : TW(0), st, seed);
+                     cr ? dtdy1d_y(ic, jc - 1) : TW(0), st);
     };
     auto y2 = [&](int k, State& st) {
         const int jc = 1 + k / (NX - 2), ic = 1 + k % (NX - 2);
@@ -599,7 +423,6 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
                 { const int kk = (r - 1) * (NX - 1) + ic - 1; if (tflag[kk]) v = v - (double)Tt[(2 * MEQN + m) * NI + kk]; }
                 g = g + v;
             }
-            if (m == 0 && ((jc == MBC && (wallf & 4)) || (jc == MY + MBC && (wallf & 8)))) g = 0.0;
             GMs[m * NXY + c] = g;
             GPs[m * NXY + c] = g;
         }
@@ -608,9 +431,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     auto y3 = [&](int c) {
         const int jc = c / NX, ic = c % NX;
         if (jc < 1) return;
-        const bool wall_edge = (ic == MBC && (wallf & 1)) || (ic == MX + MBC && (wallf & 2));
         for (int m = 0; m < MEQN; m++) {
-            if (m == 0 && wall_edge) continue;
             double fm = FMs[m * NXY + c], fp = FPs[m * NXY + c];
             if (ic - 1 >= 1 && ic - 1 <= NX - 2) {
                 const int col = ic - 1;
@@ -634,13 +455,8 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     // =================== x-sweeps (clawpack46_step2.f:113-167) ===================
     State st;
     if (bcc) { fix_corners(0); __syncthreads(); }
-    cell_fluxes(1);
-    if constexpr (RP::EXACT64 && F32) { __syncthreads(); }   // the exact solver reads the cell fluxes
-    {
-        const double seed = (RP::EXACT64 && sp.mlp) ? mlp_seed(1, tid < G::NIX ? tid : -1) : 0.0;
-        if (REG) { if (tid < G::NIX) x1(tid, st, seed); }
-        else for (int k = tid; k < G::NIX; k += NT) x1(k, st, 0.0);
-    }
+    if (REG) { if (tid < G::NIX) x1(tid, st); }
+    else for (int k = tid; k < G::NIX; k += NT) x1(k, st);
     __syncthreads();
     if (REG) { if (tid < G::NIX) x2(tid, st); }
     else for (int k = tid; k < G::NIX; k += NT) { restore(k, st); x2(k, st); }
@@ -648,14 +464,9 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     if (bcc) { fix_corners(1); __syncthreads(); }
     // X3 and the y-sweep normal solves touch disjoint data: one phase
     for (int c = tid; c < NXY; c += NT) x3(c);
-    cell_fluxes(2);
-    if constexpr (RP::EXACT64 && F32) { __syncthreads(); }
     // =================== y-sweeps (clawpack46_step2.f:182-236) ===================
-    {
-        const double seed = (RP::EXACT64 && sp.mlp) ? mlp_seed(2, tid < G::NIY ? tid : -1) : 0.0;
-        if (REG) { if (tid < G::NIY) y1(tid, st, seed); }
-        else for (int k = tid; k < G::NIY; k += NT) y1(k, st, 0.0);
-    }
+    if (REG) { if (tid < G::NIY) y1(tid, st); }
+    else for (int k = tid; k < G::NIY; k += NT) y1(k, st);
     __syncthreads();
     if (REG) { if (tid < G::NIY) y2(tid, st); }
     else for (int k = tid; k < G::NIY; k += NT) { restore(k, st); y2(k, st); }
@@ -754,22 +565,11 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
             atomicMax(cfl_bits + pd.inst, bits);
         }
     }
-    if constexpr (RP::EXACT64) {
-        if (tid < 32 && sp.newton_hist && nhist[tid]) atomicAdd(&sp.newton_hist[tid], (unsigned long long)nhist[tid]);
-    }
 }
 
 // The fused update of npatch patches starting at slot p0.  One CTA per patch, or
 // (PERSIST) a grid of a few CTAs per SM, each taking patches p0 + blockIdx.x,
 // + gridDim.x, ... in turn, its shared memory reused patch after patch.
-// Parameter block of relative patch b of a launch over lg.nlev levels.
-__device__ __forceinline__ int group_slot(const LevelGroup& lg, int b)
-{
-    int k = 0;
-    for (int i = 1; i < lg.nlev; i++) k += (b >= lg.start[i]) ? 1 : 0;
-    return lg.nlev - 1 - k;
-}
-
 template <class RP, int MX, int MY, int MBC, bool FWAVE, int NT, typename TW, int MINB = 2, bool PERSIST = false>
 __global__ void __launch_bounds__(NT, MINB)
 step2_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __restrict__ aux,
@@ -780,17 +580,16 @@ step2_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* _
     grid_launch_dependents();
     // per-launch parameters live in device memory (graph replay); a launch over
     // several levels holds one block per level, highest level first
-    __shared__ unsigned int nhist[RP::EXACT64 ? 32 : 1];
     if constexpr (!PERSIST) {
         (void)npatch;
         const int p = p0 + (int)blockIdx.x;
         const StepParams sp = spp[group_slot(lg, (int)blockIdx.x)];
-        step2_patch<RP, MX, MY, MBC, FWAVE, NT, TW>(q, qlast, aux, regs, desc, p, sp, cfl_bits, nhist);
+        step2_patch<RP, MX, MY, MBC, FWAVE, NT, TW>(q, qlast, aux, regs, desc, p, sp, cfl_bits);
     } else {
         for (int b = blockIdx.x; b < npatch; b += gridDim.x) {
             const int p = p0 + b;
             const StepParams sp = spp[group_slot(lg, b)];
-            step2_patch<RP, MX, MY, MBC, FWAVE, NT, TW>(q, qlast, aux, regs, desc, p, sp, cfl_bits, nhist);
+            step2_patch<RP, MX, MY, MBC, FWAVE, NT, TW>(q, qlast, aux, regs, desc, p, sp, cfl_bits);
             __syncthreads();   // the next patch restages the shared memory
         }
     }

@@ -1,7 +1,7 @@
 // k_step2_f64_sw.cu -- FP64 instantiations (built with -fmad=false: bitwise equal to the FP64 CPU path)
-// of the fused update for shallow water (Roe and f-wave): the patch-to-CTA variants of each patch size
-// (one CTA per patch, then the persistent forms).
-#include "k_step2_variant.cuh"
+// of the fused update for shallow water (Roe and f-wave): per patch size the variants with the MC limiter
+// fixed at compile time (k_wave.cuh), then those for any method.
+#include "k_wave.cuh"
 #include "fc2d_b200.h"
 
 namespace fcb {
@@ -9,30 +9,26 @@ namespace fcb {
 const Step2Variant* step2_table_f64_sw(int* n)
 {
     static const Step2Variant table[] = {
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 16, false, 352, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 16, false, 416, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 16, false, 352, 1, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 16, false, 256, 3, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 8, false, 160, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 8, false, 128, 4, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 8, false, 160, 4, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 8, false, 64, 8, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 16, true, 352, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 16, true, 416, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 16, true, 352, 1, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 16, true, 256, 3, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 8, true, 160, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 8, true, 128, 4, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 8, true, 160, 4, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 8, true, 64, 8, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 16, false, 352, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 16, false, 352, 1, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 8, false, 160, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, RPShallowRoe, 8, false, 128, 4, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 16, true, 352, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 16, true, 352, 1, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 8, true, 160, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, RPShallowFWave, 8, true, 128, 4, double),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 2, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 384, 2, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 1, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 2, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 1, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 4, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 5, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 6, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 4, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 6, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 2, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 384, 2, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 1, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 2, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 1, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 4, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 5, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 6, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 4, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 6, double, 0),
     };
     *n = (int)(sizeof(table) / sizeof(table[0]));
     return table;

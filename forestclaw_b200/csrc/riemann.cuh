@@ -1,4 +1,5 @@
-// riemann.cuh -- __device__ Riemann solvers of the B200 package.
+// riemann.cuh -- __device__ Riemann solvers of the advection apps, limiters, and the pressure
+// function of the exact Euler solver (the flux-form systems' solvers: wave_solvers.cuh).
 //
 // Each solver is a struct with compile-time sizes and two device functions that
 // act on ONE interface (the per-interface body of the reference's loop over
@@ -22,20 +23,26 @@ template <typename T> __device__ __forceinline__ T dmin1(T a, T b) { return a < 
 template <typename T> __device__ __forceinline__ T dmax1(T a, T b) { return a > b ? a : b; }
 template <typename T> __device__ __forceinline__ T sgn1(T x) { return copysign(T(1), x); }
 
+// Correctly rounded, uncontracted multiply / add.  The FP32-wave units are built with
+// FMA contraction; the second-order correction must not be contracted, or the
+// exactly opposite terms of the waves at a reflecting wall leave the rounding
+// error of one product as a flux through the wall.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+
 // ---------------------------------------------------------------------------
 // Scalar advection with edge velocities in aux(:,:,1:2).
 // applications/clawpack/advection/2d/all/clawpack46_rpn2adv.f, clawpack46_rpt2adv.f
 // ---------------------------------------------------------------------------
 struct RPAdvection {
     static constexpr int MEQN = 1, MWAVES = 1, MAUX = 2, NEXTRA = 1;
-    static constexpr bool CONS_FLUX = false, EXACT64 = false;
-    __device__ static void flux64(int ixy, const double* q, double grav, double* f) { (void)ixy; (void)grav; f[0] = q[0]; }
     // FP64 Godunov split for the FP32-wave path
-    __device__ static void godunov64(int ixy, const double* qL, const double* qR, const double* aL, const double* aR,
-                                     const double* fL, const double* fR, const float* ap32, double* am, double* ap,
-                                     double grav)
+    __device__ static void godunov64(int ixy, const double* qL, const double* qR, const double* aR, double* am, double* ap)
     {
-        (void)aL; (void)fL; (void)fR; (void)ap32; (void)grav;
         const double s = aR[ixy - 1], d = qR[0] - qL[0];
         am[0] = 0.0 + dmin1(s, 0.0) * d;
         ap[0] = 0.0 + dmax1(s, 0.0) * d;
@@ -71,13 +78,8 @@ struct RPAdvection {
 // ---------------------------------------------------------------------------
 struct RPAdvectionManifold {
     static constexpr int MEQN = 1, MWAVES = 1, MAUX = 3, NEXTRA = 1;
-    static constexpr bool CONS_FLUX = false, EXACT64 = false;
-    __device__ static void flux64(int ixy, const double* q, double grav, double* f) { (void)ixy; (void)grav; f[0] = q[0]; }
-    __device__ static void godunov64(int ixy, const double* qL, const double* qR, const double* aL, const double* aR,
-                                     const double* fL, const double* fR, const float* ap32, double* am, double* ap,
-                                     double grav)
+    __device__ static void godunov64(int ixy, const double* qL, const double* qR, const double* aR, double* am, double* ap)
     {
-        (void)aL; (void)fL; (void)fR; (void)ap32; (void)grav;
         const double s = aR[ixy], d = qR[0] - qL[0];
         am[0] = dmin1(s, 0.0) * d;
         ap[0] = dmax1(s, 0.0) * d;
@@ -105,283 +107,12 @@ struct RPAdvectionManifold {
 };
 
 // ---------------------------------------------------------------------------
-// Shallow water, Roe solver with Harten-Hyman entropy fix.
-// applications/clawpack/shallow/2d/rp/clawpack46_rpn2.f:1-247, clawpack46_rpt2.f:248-321
-// extra = Roe averages (u, v, a) of the interface (the common block /comroe/).
+// 2D Euler, exact Riemann solver (no counterpart in the reference): the pressure function,
+// fluxes and star pressure.  Newton iteration on p* (Toro, Riemann Solvers and Numerical
+// Methods for Fluid Dynamics, ch. 4: pressure functions 4.6-4.7, PVRS start 4.47, sampling
+// 4.5).  The interface solve is WaveEulerExact (wave_solvers.cuh).
 // ---------------------------------------------------------------------------
-struct RPShallowRoe {
-    static constexpr int MEQN = 3, MWAVES = 3, MAUX = 0, NEXTRA = 3;
-    static constexpr bool CONS_FLUX = true, EXACT64 = false;
-    static constexpr bool DEPTH = true;     // field 0 is a depth: negative values are a failure
-    // normal flux in direction ixy, FP64 (one division per cell)
-    __device__ static void flux64(int ixy, const double* q, double grav, double* f)
-    {
-        const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
-        const double h = q[0], inv = 1.0 / h;
-        f[0] = q[mu];
-        f[mu] = q[mu] * q[mu] * inv + 0.5 * grav * h * h;
-        f[mv] = q[mu] * q[mv] * inv;
-    }
-    // amdq as the FP64 remainder of the flux difference: amdq + apdq = f(qR) - f(qL)
-    __device__ static void godunov64(int ixy, const double* qL, const double* qR, const double* aL, const double* aR,
-                                     const double* fL, const double* fR, const float* ap32, double* am, double* ap,
-                                     double grav)
-    {
-        (void)ixy; (void)qL; (void)qR; (void)aL; (void)aR; (void)grav;
-        for (int m = 0; m < 3; m++) { ap[m] = (double)ap32[m]; am[m] = (fR[m] - fL[m]) - ap[m]; }
-    }
-    template <typename T>
-    __device__ static void rpn2(int ixy, const T* qL, const T* qR, const T* auxL, const T* auxR,
-                                T wave[MWAVES][MEQN], T s[MWAVES], T amdq[MEQN], T apdq[MEQN],
-                                T extra[NEXTRA], T grav)
-    {
-        (void)auxL; (void)auxR;
-        const int mu = (ixy == 1) ? 1 : 2;   // 0-based component of the normal momentum
-        const int mv = (ixy == 1) ? 2 : 1;
-        // :91-99
-        T h = (qL[0] + qR[0]) / T(2);
-        T hsqrtl = sqrt(qL[0]);
-        T hsqrtr = sqrt(qR[0]);
-        T hsq2 = hsqrtl + hsqrtr;
-        T u = (qL[mu] / hsqrtl + qR[mu] / hsqrtr) / hsq2;
-        T v = (qL[mv] / hsqrtl + qR[mv] / hsqrtr) / hsq2;
-        T a = sqrt(grav * h);
-        extra[0] = u; extra[1] = v; extra[2] = a;
-        // :105-129
-        T d1 = qR[0] - qL[0];
-        T d2 = qR[mu] - qL[mu];
-        T d3 = qR[mv] - qL[mv];
-        T a1 = ((u + a) * d1 - d2) / (T(2) * a);
-        T a2 = -(v * d1) + d3;
-        T a3 = (-((u - a) * d1) + d2) / (T(2) * a);
-        wave[0][0] = a1; wave[0][mu] = a1 * (u - a); wave[0][mv] = a1 * v; s[0] = u - a;
-        wave[1][0] = T(0); wave[1][mu] = T(0); wave[1][mv] = a2; s[1] = u;
-        wave[2][0] = a3; wave[2][mu] = a3 * (u + a); wave[2][mv] = a3 * v; s[2] = u + a;
-        // entropy fix :170-229
-        do {
-            T him1 = qL[0];
-            T s0 = qL[mu] / him1 - sqrt(grav * him1);
-            if (s0 > T(0) && s[0] > T(0)) {
-                amdq[0] = T(0); amdq[1] = T(0); amdq[2] = T(0);
-                break;
-            }
-            T h1 = qL[0] + wave[0][0];
-            T hu1 = qL[mu] + wave[0][mu];
-            T s1 = hu1 / h1 - sqrt(grav * h1);
-            T sfract;
-            if (s0 < T(0) && s1 > T(0)) sfract = s0 * ((s1 - s[0]) / (s1 - s0));
-            else if (s[0] < T(0)) sfract = s[0];
-            else sfract = T(0);
-            for (int m = 0; m < 3; m++) amdq[m] = sfract * wave[0][m];
-            if (s[1] > T(0)) break;
-            for (int m = 0; m < 3; m++) amdq[m] = amdq[m] + s[1] * wave[1][m];
-            T hi = qR[0];
-            T s03 = qR[mu] / hi + sqrt(grav * hi);
-            T h3 = qR[0] - wave[2][0];
-            T hu3 = qR[mu] - wave[2][mu];
-            T s3 = hu3 / h3 + sqrt(grav * h3);
-            if (s3 < T(0) && s03 > T(0)) sfract = s3 * ((s03 - s[2]) / (s03 - s3));
-            else if (s[2] < T(0)) sfract = s[2];
-            else break;
-            for (int m = 0; m < 3; m++) amdq[m] = amdq[m] + sfract * wave[2][m];
-        } while (0);
-        // :234-242
-        for (int m = 0; m < 3; m++) {
-            T df = T(0);
-            for (int mw = 0; mw < 3; mw++) df = df + s[mw] * wave[mw][m];
-            apdq[m] = df - amdq[m];
-        }
-    }
-    template <typename T>
-    __device__ static void rpt2(int ixy, int imp, const T* qL, const T* qR, const T* aux1, const T* aux2,
-                                const T* aux3, const T extra[NEXTRA], const T* asdq, T* bm, T* bp, T grav, T drytol)
-    {
-        (void)imp; (void)qL; (void)qR; (void)aux1; (void)aux2; (void)aux3; (void)grav; (void)drytol;
-        const int mu = (ixy == 1) ? 1 : 2;
-        const int mv = (ixy == 1) ? 2 : 1;
-        T u = extra[0], v = extra[1], a = extra[2];
-        T a1 = ((v + a) * asdq[0] - asdq[mv]) / (T(2) * a);
-        T a2 = asdq[mu] - u * asdq[0];
-        T a3 = (-((v - a) * asdq[0]) + asdq[mv]) / (T(2) * a);
-        T wb[3][3];   // wb[mw][m]
-        T sb[3];
-        wb[0][0] = a1; wb[0][mu] = a1 * u; wb[0][mv] = a1 * (v - a); sb[0] = v - a;
-        wb[1][0] = T(0); wb[1][mu] = a2; wb[1][mv] = T(0); sb[1] = v;
-        wb[2][0] = a3; wb[2][mu] = a3 * u; wb[2][mv] = a3 * (v + a); sb[2] = v + a;
-        for (int m = 0; m < 3; m++) {
-            T b1 = T(0), b2 = T(0);
-            for (int mw = 0; mw < 3; mw++) {
-                b1 = b1 + dmin1(sb[mw], T(0)) * wb[mw][m];
-                b2 = b2 + dmax1(sb[mw], T(0)) * wb[mw][m];
-            }
-            bm[m] = b1; bp[m] = b2;
-        }
-    }
-};
-
-// ---------------------------------------------------------------------------
-// Shallow water f-waves with bathymetry b = aux(:,:,1).
-// applications/clawpack/shallow/2d/rp/rpn2_tsunami.f90:3-222, rpt2_tsunami.f90:3-170
-// ---------------------------------------------------------------------------
-struct RPShallowFWave {
-    static constexpr int MEQN = 3, MWAVES = 3, MAUX = 1, NEXTRA = 1;
-    static constexpr bool CONS_FLUX = true, EXACT64 = false;
-    static constexpr bool DEPTH = true;
-    // normal flux in direction ixy, FP64 (one division per cell)
-    __device__ static void flux64(int ixy, const double* q, double grav, double* f)
-    {
-        const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
-        const double h = q[0], inv = 1.0 / h;
-        f[0] = q[mu];
-        f[mu] = q[mu] * q[mu] * inv + 0.5 * grav * h * h;
-        f[mv] = q[mu] * q[mv] * inv;
-    }
-    // f-waves sum to the flux difference plus the bathymetry source g*hbar*(bR-bL)
-    __device__ static void godunov64(int ixy, const double* qL, const double* qR, const double* aL, const double* aR,
-                                     const double* fL, const double* fR, const float* ap32, double* am, double* ap,
-                                     double grav)
-    {
-        const int mu = (ixy == 1) ? 1 : 2;
-        for (int m = 0; m < 3; m++) {
-            double fd = fR[m] - fL[m];
-            if (m == mu) fd = fd + grav * (0.5 * (qR[0] + qL[0])) * (aR[0] - aL[0]);
-            ap[m] = (double)ap32[m];
-            am[m] = fd - ap[m];
-        }
-    }
-    template <typename T>
-    __device__ static void rpn2(int ixy, const T* qL, const T* qR, const T* auxL, const T* auxR,
-                                T fwave[MWAVES][MEQN], T s[MWAVES], T amdq[MEQN], T apdq[MEQN],
-                                T extra[NEXTRA], T grav)
-    {
-        (void)extra;
-        const int mu = (ixy == 1) ? 1 : 2;
-        const int mv = (ixy == 1) ? 2 : 1;
-        T hL = qL[0], hR = qR[0];
-        T huL = qL[mu], huR = qR[mu];
-        T bL = auxL[0], bR = auxR[0];
-        T hvL = qL[mv], hvR = qR[mv];
-        T uR = huR / hR, vR = hvR / hR;
-        T phiR = T(0.5) * grav * (hR * hR) + (huR * huR) / hR;
-        T uL = huL / hL, vL = hvL / hL;
-        T phiL = T(0.5) * grav * (hL * hL) + (huL * huL) / hL;
-        T uhat = (sqrt(grav * hL) * uL + sqrt(grav * hR) * uR) / (sqrt(grav * hR) + sqrt(grav * hL));
-        T chat = sqrt(grav * T(0.5) * (hR + hL));
-        T hbar = T(0.5) * (hR + hL);
-        T fd1 = (hR * uR) - (hL * uL);
-        T fd2 = phiR - phiL + grav * hbar * (bR - bL);
-        T fd3 = hR * uR * vR - hL * uL * vL;
-        T s1 = fmin(uL - sqrt(grav * hL), uhat - chat);
-        T s3 = fmax(uR + sqrt(grav * hR), uhat + chat);
-        T s2 = T(0.5) * (s1 + s3);
-        T b1 = -(fd2 - s3 * fd1) / (s3 - s1);
-        T b3 = (fd2 - s1 * fd1) / (s3 - s1);
-        T b2 = fd3 - b1 * vL - b3 * vR;
-        T fw[3][3];   // fw[row][wave], rows (h, normal, transverse)
-        fw[0][0] = b1; fw[1][0] = b1 * s1; fw[2][0] = b1 * vL;
-        fw[0][1] = T(0); fw[1][1] = T(0); fw[2][1] = b2;
-        fw[0][2] = b3; fw[1][2] = b3 * s3; fw[2][2] = b3 * vR;
-        s[0] = s1; s[1] = s2; s[2] = s3;
-        for (int mw = 0; mw < 3; mw++) {
-            fwave[mw][0] = fw[0][mw];
-            fwave[mw][mu] = fw[1][mw];
-            fwave[mw][mv] = fw[2][mw];
-        }
-        T szm[3], szp[3];
-        for (int mw = 0; mw < 3; mw++) {
-            T z = sgn1(s[mw]);
-            szm[mw] = (T(1) - z) / T(2);
-            szp[mw] = (T(1) + z) / T(2);
-        }
-        for (int m = 0; m < 3; m++) {
-            T am = szm[0] * fwave[0][m];
-            am = am + szm[1] * fwave[1][m];
-            am = am + szm[2] * fwave[2][m];
-            T ap = szp[0] * fwave[0][m];
-            ap = ap + szp[1] * fwave[1][m];
-            ap = ap + szp[2] * fwave[2][m];
-            amdq[m] = am; apdq[m] = ap;
-        }
-    }
-    template <typename T>
-    __device__ static void rpt2(int ixy, int imp, const T* qL, const T* qR, const T* aux1, const T* aux2,
-                                const T* aux3, const T extra[NEXTRA], const T* asdq, T* bm, T* bp, T g, T tol)
-    {
-        (void)extra;
-        const int mu = (ixy == 1) ? 1 : 2;
-        const int mv = (ixy == 1) ? 2 : 1;
-        T hl = qL[0], hr = qR[0];
-        T hul = qL[mu], hur = qR[mu];
-        T hvl = qL[mv], hvr = qR[mv];
-        T ul, vl, ur, vr;
-        if (hl < tol) { hl = T(0); ul = T(0); vl = T(0); } else { ul = hul / hl; vl = hvl / hl; }
-        if (hr < tol) { hr = T(0); ur = T(0); vr = T(0); } else { ur = hur / hr; vr = hvr / hr; }
-        T sv[3] = {T(0), T(0), T(0)}, beta[3] = {T(0), T(0), T(0)};
-        T r[3][3] = {{T(0), T(0), T(0)}, {T(0), T(0), T(0)}, {T(0), T(0), T(0)}};   // r[m][mw]
-        bool skip = (hl <= tol && hr <= tol);
-        if (!skip) {
-            T eta = (imp == 1) ? qL[0] + aux2[0] : qR[0] + aux2[0];
-            if (eta < fmax(aux1[0], aux3[0])) skip = true;
-        }
-        if (!skip) {
-            T vhat = (vr * sqrt(hr)) / (sqrt(hr) + sqrt(hl)) + (vl * sqrt(hl)) / (sqrt(hr) + sqrt(hl));
-            T uhat = (ur * sqrt(hr)) / (sqrt(hr) + sqrt(hl)) + (ul * sqrt(hl)) / (sqrt(hr) + sqrt(hl));
-            T hhat = (hr + hl) / T(2);
-            T roe1 = vhat - sqrt(g * hhat);
-            T roe3 = vhat + sqrt(g * hhat);
-            T s1l = vl - sqrt(g * hl);
-            T s3r = vr + sqrt(g * hr);
-            T s1 = fmin(roe1, s1l);
-            T s3 = fmax(roe3, s3r);
-            T s2 = uhat;
-            sv[0] = s1; sv[1] = s2; sv[2] = s3;
-            T delf1 = asdq[0], delf2 = asdq[mu], delf3 = asdq[mv];
-            beta[0] = (s3 * delf1 / (s3 - s1)) - (delf3 / (s3 - s1));
-            beta[1] = -(s2 * delf1) + delf2;
-            beta[2] = (delf3 / (s3 - s1)) - (s1 * delf1 / (s3 - s1));
-            r[0][0] = T(1); r[mu][0] = s2; r[mv][0] = s1;
-            r[0][1] = T(0); r[mu][1] = T(1); r[mv][1] = T(0);
-            r[0][2] = T(1); r[mu][2] = s2; r[mv][2] = s3;
-        }
-        T szm[3], szp[3];
-        for (int mw = 0; mw < 3; mw++) {
-            T z = sgn1(sv[mw]);
-            szm[mw] = (T(1) - z) / T(2) * sv[mw] * beta[mw];
-            szp[mw] = (T(1) + z) / T(2) * sv[mw] * beta[mw];
-        }
-        for (int m = 0; m < 3; m++) {
-            T b1 = szm[0] * r[m][0];
-            b1 = b1 + szm[1] * r[m][1];
-            b1 = b1 + szm[2] * r[m][2];
-            T b2 = szp[0] * r[m][0];
-            b2 = b2 + szp[1] * r[m][1];
-            b2 = b2 + szp[2] * r[m][2];
-            bm[m] = b1; bp[m] = b2;
-        }
-    }
-};
-
-
-// ---------------------------------------------------------------------------
-// 2D Euler, exact Riemann solver (no counterpart in the reference).
-// Newton iteration on p* (Toro, Riemann Solvers and Numerical Methods for
-// Fluid Dynamics, ch. 4: pressure functions 4.6-4.7, PVRS start 4.47, sampling
-// 4.5), always in FP64:
-//   amdq = F(q0) - F(qL), apdq = F(qR) - F(q0), q0 the Godunov state at x/t = 0,
-//   waves w1 = q*L - qL, w2 = q*R - q*L, w3 = qR - q*R,
-//   speeds s1 = left shock speed or rarefaction head uL - aL, s2 = u*,
-//          s3 = right shock speed or rarefaction head uR + aR.
-// The Roe averages of clawpack46_rpn2_euler4.f:83-100 are returned in extra for
-// the transverse solver clawpack46_rpt2_euler4.f:56-94.
-// EXACT64: the kernel calls solve64 with FP64 states and keeps amdq/apdq in FP64
-// in every precision; only the waves, speeds and transverse split use TW.
-// ---------------------------------------------------------------------------
-struct EulerParams { double gam, tol, seed; };
-
 struct RPEulerExact {
-    static constexpr int MEQN = 4, MWAVES = 3, MAUX = 0, NEXTRA = 5;
-    static constexpr bool CONS_FLUX = true, EXACT64 = true;
-
     __device__ static void prefun(double g1, double g4, double g5, double g6, double p, double rk, double pk,
                                   double ak, double& f, double& fd)
     {
@@ -491,323 +222,6 @@ struct RPEulerExact {
     }
     // Returned with the iteration count when Newton converged neither from the seed nor from PVRS.
     static constexpr int NEWTON_FAILED = 0x100;
-    // One interface, FP64.  w[mw][m], am/ap in natural component order.
-    // Returns the Newton iteration count.
-    __device__ static int solve64(int ixy, const double* qL, const double* qR, const EulerParams& ep,
-                                  double w[3][4], double s[3], double* am, double* ap, double* ex)
-    {
-        const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
-        const double gam = ep.gam, gamma1 = gam - 1.0;
-        // Roe averages (clawpack46_rpn2_euler4.f:84-99)
-        {
-            const double rhsqrtl = sqrt(qL[0]);
-            const double rhsqrtr = sqrt(qR[0]);
-            const double pl = gamma1 * (qL[3] - 0.5 * (qL[1] * qL[1] + qL[2] * qL[2]) / qL[0]);
-            const double pr = gamma1 * (qR[3] - 0.5 * (qR[1] * qR[1] + qR[2] * qR[2]) / qR[0]);
-            const double rhsq2 = rhsqrtl + rhsqrtr;
-            const double u = (qL[mu] / rhsqrtl + qR[mu] / rhsqrtr) / rhsq2;
-            const double v = (qL[mv] / rhsqrtl + qR[mv] / rhsqrtr) / rhsq2;
-            const double enth = ((qL[3] + pl) / rhsqrtl + (qR[3] + pr) / rhsqrtr) / rhsq2;
-            const double u2v2 = u * u + v * v;
-            const double a2 = gamma1 * (enth - 0.5 * u2v2);
-            ex[0] = u; ex[1] = v; ex[2] = enth; ex[3] = sqrt(a2); ex[4] = gamma1 / a2;
-        }
-        const double g1 = (gam - 1.0) / (2.0 * gam), g2 = (gam + 1.0) / (2.0 * gam);
-        const double g3 = 2.0 * gam / (gam - 1.0), g4 = 2.0 / (gam - 1.0), g5 = 2.0 / (gam + 1.0);
-        const double g6 = (gam - 1.0) / (gam + 1.0), g7 = (gam - 1.0) / 2.0;
-        const Prim P = prim(ixy, qL, qR, gam);
-        const double du = P.ur - P.ul;
-        const double tolpre = 1.0e-6;
-        double p;
-        if (ep.seed > 0.0 && isfinite(ep.seed)) p = ep.seed;
-        else {
-            const double ppv = 0.5 * (P.pl + P.pr) - 0.125 * du * (P.rl + P.rr) * (P.al + P.ar);
-            p = ppv > tolpre ? ppv : tolpre;
-        }
-        double fl = 0.0, fr = 0.0, fdl, fdr;
-        int it = 0;
-        bool ok = true;
-        if (P.pl == P.pr && P.ul == P.ur) {
-            // no pressure or normal-velocity jump: p* = p, u* = u exactly (the first
-            // Newton step's values, bit for bit), no iteration
-            p = P.pl;
-        } else {
-            // Newton from the seed; where it does not converge, again from PVRS
-            const bool seeded = ep.seed > 0.0 && isfinite(ep.seed);
-            ok = false;
-            for (int pass = 0; pass < (seeded ? 2 : 1) && !ok; pass++) {
-                if (pass == 1) {
-                    const double ppv = 0.5 * (P.pl + P.pr) - 0.125 * du * (P.rl + P.rr) * (P.al + P.ar);
-                    p = ppv > tolpre ? ppv : tolpre;
-                }
-                for (int k = 1; k <= 64; k++) {
-                    prefun(g1, g4, g5, g6, p, P.rl, P.pl, P.al, fl, fdl);
-                    prefun(g1, g4, g5, g6, p, P.rr, P.pr, P.ar, fr, fdr);
-                    double pn = p - (fl + fr + du) / (fdl + fdr);
-                    if (pn < 0.0) pn = tolpre;
-                    const double change = 2.0 * fabs(pn - p) / (pn + p);
-                    p = pn;
-                    it++;
-                    if (change <= ep.tol) { ok = true; break; }
-                }
-                ok = ok && isfinite(p);
-            }
-            if (it > 64) it = 64;
-        }
-        const double ps = p;
-        const double us = 0.5 * (P.ul + P.ur) + 0.5 * (fr - fl);
-        // star densities and sound speeds (p* = pK: rhoK, aK exactly, as log 1 = 0, exp 0 = 1)
-        double rsl, rsr, asl, asr;
-        if (ps > P.pl) { const double q = ps / P.pl; rsl = P.rl * ((q + g6) / (g6 * q + 1.0)); asl = sqrt(gam * ps / rsl); }
-        else if (ps == P.pl) { rsl = P.rl; asl = P.al; }
-        else { const double lq = fcb_log(ps / P.pl); rsl = P.rl * fcb_exp(lq / gam); asl = P.al * fcb_exp(g1 * lq); }
-        if (ps > P.pr) { const double q = ps / P.pr; rsr = P.rr * ((q + g6) / (g6 * q + 1.0)); asr = sqrt(gam * ps / rsr); }
-        else if (ps == P.pr) { rsr = P.rr; asr = P.ar; }
-        else { const double lq = fcb_log(ps / P.pr); rsr = P.rr * fcb_exp(lq / gam); asr = P.ar * fcb_exp(g1 * lq); }
-        const double shl = P.ul - P.al, shr = P.ur + P.ar;
-        double sl, sr;
-        if (ps > P.pl) sl = P.ul - P.al * sqrt(g2 * (ps / P.pl) + g1); else sl = shl;
-        if (ps > P.pr) sr = P.ur + P.ar * sqrt(g2 * (ps / P.pr) + g1); else sr = shr;
-        s[0] = sl; s[1] = us; s[2] = sr;
-        const double esl = ps / gamma1 + 0.5 * rsl * (us * us + P.vl * P.vl);
-        const double esr = ps / gamma1 + 0.5 * rsr * (us * us + P.vr * P.vr);
-        // waves in (rho, m_n, m_t, E) order, stored at the natural components
-        const double qln[4] = {qL[0], qL[mu], qL[mv], qL[3]}, qrn[4] = {qR[0], qR[mu], qR[mv], qR[3]};
-        const double qsl[4] = {rsl, rsl * us, rsl * P.vl, esl};
-        const double qsr[4] = {rsr, rsr * us, rsr * P.vr, esr};
-        const int comp[4] = {0, mu, mv, 3};
-        for (int k = 0; k < 4; k++) {
-            w[0][comp[k]] = qsl[k] - qln[k];
-            w[1][comp[k]] = qsr[k] - qsl[k];
-            w[2][comp[k]] = qrn[k] - qsr[k];
-        }
-        // Godunov state at x/t = 0
-        double r0, u0, v0, p0, e0;
-        int which;
-        if (0.0 <= us) {
-            v0 = P.vl;
-            if (ps > P.pl) which = (0.0 <= sl) ? 0 : 1;
-            else if (0.0 <= shl) which = 0;
-            else which = (0.0 > us - asl) ? 1 : 2;
-        } else {
-            v0 = P.vr;
-            if (ps > P.pr) which = (0.0 >= sr) ? 4 : 3;
-            else if (0.0 >= shr) which = 4;
-            else which = (0.0 < us + asr) ? 3 : 5;
-        }
-        if (which == 0) { r0 = P.rl; u0 = P.ul; p0 = P.pl; e0 = qL[3]; }
-        else if (which == 4) { r0 = P.rr; u0 = P.ur; p0 = P.pr; e0 = qR[3]; }
-        else if (which == 1) { r0 = rsl; u0 = us; p0 = ps; e0 = esl; }
-        else if (which == 3) { r0 = rsr; u0 = us; p0 = ps; e0 = esr; }
-        else if (which == 2) {
-            const double c = g5 + (g6 / P.al) * P.ul;
-            const double lc = fcb_log(c);
-            r0 = P.rl * fcb_exp(g4 * lc);
-            u0 = g5 * (P.al + g7 * P.ul);
-            p0 = P.pl * fcb_exp(g3 * lc);
-            e0 = p0 / gamma1 + 0.5 * r0 * (u0 * u0 + v0 * v0);
-        } else {
-            const double c = g5 - (g6 / P.ar) * P.ur;
-            const double lc = fcb_log(c);
-            r0 = P.rr * fcb_exp(g4 * lc);
-            u0 = g5 * (-P.ar + g7 * P.ur);
-            p0 = P.pr * fcb_exp(g3 * lc);
-            e0 = p0 / gamma1 + 0.5 * r0 * (u0 * u0 + v0 * v0);
-        }
-        double f0[4], flv[4], frv[4];
-        eflux(r0, u0, v0, p0, e0, f0);
-        eflux(P.rl, P.ul, P.vl, P.pl, qL[3], flv);
-        eflux(P.rr, P.ur, P.vr, P.pr, qR[3], frv);
-        for (int k = 0; k < 4; k++) { am[comp[k]] = f0[k] - flv[k]; ap[comp[k]] = frv[k] - f0[k]; }
-        return it | (ok ? 0 : NEWTON_FAILED);
-    }
-    // FP32-wave form of solve64.  Primitive states, Roe averages, the Newton
-    // iteration on p* (only where p or u jumps), star states, the Godunov state and
-    // the waves in FP32.  The Godunov flux f0 is one FP32
-    // value per interface, so amdq = f0 - F(qL) and apdq = F(qR) - f0 with the FP64
-    // cell fluxes of flxL/flxR keep the update conservative in FP64.
-    __device__ static int solve_mixed(int ixy, const float* qL, const float* qR, const double* qL64,
-                                      const double* qR64, const double* flxL, const double* flxR,
-                                      const EulerParams& ep, float w[3][4], float s[3], double* am, double* ap,
-                                      float* ex)
-    {
-        const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
-        const float gam = (float)ep.gam, gamma1 = gam - 1.0f;
-        const float g1 = (gam - 1.0f) / (2.0f * gam), g2 = (gam + 1.0f) / (2.0f * gam);
-        const float g3 = 2.0f * gam / (gam - 1.0f), g4 = 2.0f / (gam - 1.0f), g5 = 2.0f / (gam + 1.0f);
-        const float g6 = (gam - 1.0f) / (gam + 1.0f), g7 = (gam - 1.0f) / 2.0f;
-        {   // Roe averages for rpt2
-            const float rhsqrtl = sqrtf(qL[0]), rhsqrtr = sqrtf(qR[0]);
-            const float pl = gamma1 * (qL[3] - 0.5f * (qL[1] * qL[1] + qL[2] * qL[2]) / qL[0]);
-            const float pr = gamma1 * (qR[3] - 0.5f * (qR[1] * qR[1] + qR[2] * qR[2]) / qR[0]);
-            const float rhsq2 = rhsqrtl + rhsqrtr;
-            const float u = (qL[mu] / rhsqrtl + qR[mu] / rhsqrtr) / rhsq2;
-            const float v = (qL[mv] / rhsqrtl + qR[mv] / rhsqrtr) / rhsq2;
-            const float enth = ((qL[3] + pl) / rhsqrtl + (qR[3] + pr) / rhsqrtr) / rhsq2;
-            const float a2 = gamma1 * (enth - 0.5f * (u * u + v * v));
-            ex[0] = u; ex[1] = v; ex[2] = enth; ex[3] = sqrtf(a2); ex[4] = gamma1 / a2;
-        }
-        // primitive states with correctly rounded, uncontracted operations, so the
-        // two sides of an interface between equal states compute the same values
-        auto pres = [&](const float* q) {
-            const float ke = __fdiv_rn(__fmul_rn(0.5f, __fadd_rn(__fmul_rn(q[mu], q[mu]), __fmul_rn(q[mv], q[mv]))), q[0]);
-            return __fmul_rn(gamma1, __fsub_rn(q[3], ke));
-        };
-        const float rl = qL[0], ul = __fdiv_rn(qL[mu], rl), vl = __fdiv_rn(qL[mv], rl), pl = pres(qL);
-        const float rr = qR[0], ur = __fdiv_rn(qR[mu], rr), vr = __fdiv_rn(qR[mv], rr), pr = pres(qR);
-        const float al = sqrtf(gam * pl / rl), ar = sqrtf(gam * pr / rr);
-        int it = 0;
-        bool ok = true;
-        float ps, us;
-        const bool nojump = (pl == pr && ul == ur);
-        if (nojump) {
-            ps = pl; us = ul;
-        } else {
-            // Newton on p* in FP32 from the FP32 primitive states (Toro's pressure
-            // function; the FP64 form iterates in FP64 with the deterministic exp/log).
-            // FP32 resolves p* to a few ulp, so the iteration stops at a relative change
-            // of max(tol, NEWTON_TOL32).
-            (void)qL64; (void)qR64;
-            const float du = ur - ul, tolpre = 1.0e-6f;
-            float p;
-            if (ep.seed > 0.0 && isfinite(ep.seed)) p = (float)ep.seed;
-            else {
-                const float ppv = 0.5f * (pl + pr) - 0.125f * du * (rl + rr) * (al + ar);
-                p = ppv > tolpre ? ppv : tolpre;
-            }
-            const float tol = fmaxf((float)ep.tol, NEWTON_TOL32);
-            float fl = 0.0f, fr = 0.0f, fdl, fdr;
-            // Newton from the seed; where it does not converge, again from PVRS
-            const bool seeded = ep.seed > 0.0 && isfinite(ep.seed);
-            bool conv = false;
-            for (int pass = 0; pass < (seeded ? 2 : 1) && !conv; pass++) {
-                if (pass == 1) {
-                    const float ppv = 0.5f * (pl + pr) - 0.125f * du * (rl + rr) * (al + ar);
-                    p = ppv > tolpre ? ppv : tolpre;
-                }
-                for (int k = 1; k <= 64; k++) {
-                    prefun32(g1, g4, g5, g6, p, rl, pl, al, fl, fdl);
-                    prefun32(g1, g4, g5, g6, p, rr, pr, ar, fr, fdr);
-                    float pn = p - (fl + fr + du) / (fdl + fdr);
-                    if (pn < 0.0f) pn = tolpre;
-                    const float change = 2.0f * fabsf(pn - p) / (pn + p);
-                    p = pn;
-                    it++;
-                    if (change <= tol) { conv = true; break; }
-                }
-                conv = conv && isfinite(p);
-            }
-            ok = conv;
-            if (it > 64) it = 64;
-            ps = p;
-            us = 0.5f * (ul + ur) + 0.5f * (fr - fl);
-        }
-        float rsl, rsr, asl, asr;
-        if (ps > pl) { const float q = ps / pl; rsl = rl * ((q + g6) / (g6 * q + 1.0f)); asl = sqrtf(gam * ps / rsl); }
-        else if (ps == pl) { rsl = rl; asl = al; }
-        else { const float lq = __logf(ps / pl); rsl = rl * __expf(lq / gam); asl = al * __expf(g1 * lq); }
-        if (ps > pr) { const float q = ps / pr; rsr = rr * ((q + g6) / (g6 * q + 1.0f)); asr = sqrtf(gam * ps / rsr); }
-        else if (ps == pr) { rsr = rr; asr = ar; }
-        else { const float lq = __logf(ps / pr); rsr = rr * __expf(lq / gam); asr = ar * __expf(g1 * lq); }
-        const float shl = ul - al, shr = ur + ar;
-        const float sl = (ps > pl) ? ul - al * sqrtf(g2 * (ps / pl) + g1) : shl;
-        const float sr = (ps > pr) ? ur + ar * sqrtf(g2 * (ps / pr) + g1) : shr;
-        s[0] = sl; s[1] = us; s[2] = sr;
-        const float esl = ps / gamma1 + 0.5f * rsl * (us * us + vl * vl);
-        const float esr = ps / gamma1 + 0.5f * rsr * (us * us + vr * vr);
-        const float qln[4] = {qL[0], qL[mu], qL[mv], qL[3]}, qrn[4] = {qR[0], qR[mu], qR[mv], qR[3]};
-        const float qsl[4] = {rsl, rsl * us, rsl * vl, esl};
-        const float qsr[4] = {rsr, rsr * us, rsr * vr, esr};
-        const int comp[4] = {0, mu, mv, 3};
-        for (int k = 0; k < 4; k++) {
-            if (nojump) {   // the star states are the outer states: only the contact/shear wave
-                w[0][comp[k]] = 0.0f;
-                w[1][comp[k]] = qrn[k] - qln[k];
-                w[2][comp[k]] = 0.0f;
-            } else {
-                w[0][comp[k]] = qsl[k] - qln[k];
-                w[1][comp[k]] = qsr[k] - qsl[k];
-                w[2][comp[k]] = qrn[k] - qsr[k];
-            }
-        }
-        float r0, u0, v0, p0, e0;
-        int which;
-        if (0.0f <= us) {
-            v0 = vl;
-            if (ps > pl) which = (0.0f <= sl) ? 0 : 1;
-            else if (0.0f <= shl) which = 0;
-            else which = (0.0f > us - asl) ? 1 : 2;
-        } else {
-            v0 = vr;
-            if (ps > pr) which = (0.0f >= sr) ? 4 : 3;
-            else if (0.0f >= shr) which = 4;
-            else which = (0.0f < us + asr) ? 3 : 5;
-        }
-        if (which == 0) { r0 = rl; u0 = ul; p0 = pl; e0 = qL[3]; }
-        else if (which == 4) { r0 = rr; u0 = ur; p0 = pr; e0 = qR[3]; }
-        else if (which == 1) { r0 = rsl; u0 = us; p0 = ps; e0 = esl; }
-        else if (which == 3) { r0 = rsr; u0 = us; p0 = ps; e0 = esr; }
-        else if (which == 2) {
-            const float c = g5 + (g6 / al) * ul, lc = __logf(c);
-            r0 = rl * __expf(g4 * lc); u0 = g5 * (al + g7 * ul); p0 = pl * __expf(g3 * lc);
-            e0 = p0 / gamma1 + 0.5f * r0 * (u0 * u0 + v0 * v0);
-        } else {
-            const float c = g5 - (g6 / ar) * ur, lc = __logf(c);
-            r0 = rr * __expf(g4 * lc); u0 = g5 * (-ar + g7 * ur); p0 = pr * __expf(g3 * lc);
-            e0 = p0 / gamma1 + 0.5f * r0 * (u0 * u0 + v0 * v0);
-        }
-        if (nojump) {
-            // without a pressure / normal-velocity jump the Godunov state on the
-            // sampled side of the contact is that side's own state: its FP64 flux
-            const bool left = which <= 2;
-            for (int m = 0; m < 4; m++) {
-                am[m] = left ? 0.0 : flxR[m] - flxL[m];
-                ap[m] = left ? flxR[m] - flxL[m] : 0.0;
-            }
-            return it;
-        }
-        const float f0[4] = {r0 * u0, r0 * u0 * u0 + p0, r0 * u0 * v0, u0 * (e0 + p0)};
-        for (int k = 0; k < 4; k++) {
-            const double f = (double)f0[k];
-            am[comp[k]] = f - flxL[comp[k]];
-            ap[comp[k]] = flxR[comp[k]] - f;
-        }
-        return it | (ok ? 0 : NEWTON_FAILED);
-    }
-    // clawpack46_rpt2_euler4.f:56-94 with the Roe averages of the interface
-    template <typename T>
-    __device__ static void rpt2(int ixy, int imp, const T* qL, const T* qR, const T* aux1, const T* aux2,
-                                const T* aux3, const T extra[NEXTRA], const T* asdq, T* bm, T* bp, T grav, T drytol)
-    {
-        (void)imp; (void)qL; (void)qR; (void)aux1; (void)aux2; (void)aux3; (void)grav; (void)drytol;
-        const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
-        const T u = extra[0], v = extra[1], enth = extra[2], a = extra[3], g1a2 = extra[4];
-        const T u2v2 = u * u + v * v;
-        const T euv = enth - u2v2;
-        const T a3 = g1a2 * (euv * asdq[0] + u * asdq[mu] + v * asdq[mv] - asdq[3]);
-        const T a2 = asdq[mu] - u * asdq[0];
-        const T a4 = (asdq[mv] + (a - v) * asdq[0] - a * a3) / (T(2) * a);
-        const T a1 = asdq[0] - a3 - a4;
-        T wb[4][3], sb[3];
-        wb[0][0] = a1; wb[mu][0] = a1 * u; wb[mv][0] = a1 * (v - a); wb[3][0] = a1 * (enth - v * a); sb[0] = v - a;
-        wb[0][1] = a3; wb[mu][1] = a3 * u + a2; wb[mv][1] = a3 * v; wb[3][1] = a3 * T(0.5) * u2v2 + a2 * u; sb[1] = v;
-        wb[0][2] = a4; wb[mu][2] = a4 * u; wb[mv][2] = a4 * (v + a); wb[3][2] = a4 * (enth + v * a); sb[2] = v + a;
-        for (int m = 0; m < 4; m++) {
-            T b1 = T(0), b2 = T(0);
-            for (int mw = 0; mw < 3; mw++) {
-                b1 = b1 + (sb[mw] < T(0) ? sb[mw] : T(0)) * wb[m][mw];
-                b2 = b2 + (sb[mw] > T(0) ? sb[mw] : T(0)) * wb[m][mw];
-            }
-            bm[m] = b1; bp[m] = b2;
-        }
-    }
-    // FP64 normal flux of a cell for the FP32-wave form (gamma passed in place of grav)
-    __device__ static void flux64(int ixy, const double* q, double gam, double* f) { cons_flux(ixy - 1, q, gam, f); }
-    __device__ static void godunov64(int, const double*, const double*, const double*, const double*, const double*,
-                                     const double*, const float*, double*, double*, double) {}
-    template <typename T>
-    __device__ static void rpn2(int, const T*, const T*, const T*, const T*, T[MWAVES][MEQN], T[MWAVES], T[MEQN],
-                                T[MEQN], T[NEXTRA], T) {}
 };
 
 // clawpack46_inlinelimiter.f:59-104

@@ -76,7 +76,6 @@ constexpr int user_threads() { return MX <= 8 ? 128 : (MX <= 16 ? 352 : 512); }
 template <int MEQN_, int MWAVES_, int MAUX_, class Impl>
 struct RPUserBase {
     static constexpr int MEQN = MEQN_, MWAVES = MWAVES_, MAUX = MAUX_, NEXTRA = 1;
-    static constexpr bool CONS_FLUX = false, EXACT64 = false;
     static constexpr bool USER_HOOKS = true, AUX_BOTH = true;
     static constexpr int MA = MAUX > 0 ? MAUX : 1;
     template <typename T>
