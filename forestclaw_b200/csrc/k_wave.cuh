@@ -72,7 +72,8 @@ struct WaveGeom {
     static constexpr size_t OFF_FY = OFF_FX + FB;                // per-cell planes, then [NF][MEQN][NI] double
     static constexpr size_t OFF_RED = OFF_FY + (FB > PB ? FB : PB);
     static constexpr size_t OFF_HIST = OFF_RED + 32 * 8;
-    static constexpr size_t OFF_BAR = OFF_HIST + (RP::EXACT ? 32 * 4 : 0);
+    static constexpr size_t OFF_K = OFF_HIST + (RP::EXACT ? 32 * 4 : 0);
+    static constexpr size_t OFF_BAR = OFF_K + up16(RP::NCONST * sizeof(TW));
     static constexpr size_t OFF_W = OFF_BAR + 16;                // [NW][NI] TW
     static constexpr size_t OFF_T = OFF_W + up16((size_t)RP::NW * NI * sizeof(TW));    // [4][MEQN][NI] TW
     static constexpr size_t BYTES = OFF_T + (size_t)4 * MEQN * NI * sizeof(TW);
@@ -402,12 +403,14 @@ wave_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __
     }
     if (RP::EXACT && tid < 32) nhist[tid] = 0u;            // Newton iterations of this patch
     const StepParams* sp = spp + group_slot(lg, (int)blockIdx.x);
+    TW* konst = reinterpret_cast<TW*>(sm + G::OFF_K);
+    if constexpr (RP::NCONST > 0) { if (tid == 32) RP::constants((TW)sp->gamma, konst); }
     const PatchDesc* pd = desc + p;
     const double dx = pd->dx, dy = pd->dy;
     const double dt = sp->inst_dt ? sp->dt * sp->inst_dt[pd->inst] : sp->dt;
     // reflecting walls of this patch whose ghost cells hold mirror values (FP32-wave mass rule)
     const int wallf = F32 ? (pd->phys_mask & sp->wall_faces) : 0;
-    WP X{sm, WaveMethod<LIM>(sp), WavePar<TW>{(TW)sp->grav, (TW)sp->dry_tolerance, sp->gamma, sp->newton_tol},
+    WP X{sm, WaveMethod<LIM>(sp), WavePar<TW>{(TW)sp->grav, (TW)sp->dry_tolerance, sp->gamma, sp->newton_tol, konst},
          sp->grav, dt / dx, dt / dy, wallf};
     double* Q = X.Q();
     __syncthreads();                                        // the barrier word is initialised

@@ -27,9 +27,10 @@
 
 namespace fcb {
 
-// Scalars of a launch every solver function may need.
+// Scalars of a launch every solver function may need; k: constants of the solver in shared
+// memory (RP::NCONST of them, RP::constants), formed once per CTA.
 template <typename T>
-struct WavePar { T grav, drytol; double gamma, tol; };
+struct WavePar { T grav, drytol; double gamma, tol; const T* k; };
 
 // normal (mu) and transverse (mv) momentum component of a sweep
 template <int IXY> struct Dir { static constexpr int mu = IXY == 1 ? 1 : 2, mv = IXY == 1 ? 2 : 1; };
@@ -39,7 +40,7 @@ template <int IXY> struct Dir { static constexpr int mu = IXY == 1 ? 1 : 2, mv =
 // applications/clawpack/shallow/2d/rp/clawpack46_rpn2.f:1-247, clawpack46_rpt2.f:248-321
 // ---------------------------------------------------------------------------
 struct WaveShallowRoe {
-    static constexpr int MEQN = 3, MWAVES = 3, MAUX = 0, NPRE = 6, NW = 7, NFL = 3;
+    static constexpr int MEQN = 3, MWAVES = 3, MAUX = 0, NPRE = 6, NW = 7, NFL = 3, NCONST = 0;
     static constexpr bool FWAVE = false, DEPTH = true, EXACT = false;
     enum { P_RS = 0, P_N1 = 1, P_N2 = 2, P_U1 = 3, P_U2 = 4, P_C = 5 };   // sqrt h, (hu, hv)/sqrt h, (hu, hv)/h, sqrt gh
     template <int IXY> __host__ __device__ static constexpr int wp(int mw, int m)
@@ -183,7 +184,7 @@ struct WaveShallowRoe {
 // applications/clawpack/shallow/2d/rp/rpn2_tsunami.f90:3-222, rpt2_tsunami.f90:3-170
 // ---------------------------------------------------------------------------
 struct WaveShallowFWave {
-    static constexpr int MEQN = 3, MWAVES = 3, MAUX = 1, NPRE = 6, NW = 7, NFL = 3;
+    static constexpr int MEQN = 3, MWAVES = 3, MAUX = 1, NPRE = 6, NW = 7, NFL = 3, NCONST = 0;
     static constexpr bool FWAVE = true, DEPTH = true, EXACT = false;
     enum { P_RS = 0, P_C = 1, P_U1 = 2, P_U2 = 3, P_E1 = 4, P_E2 = 5 };   // sqrt h, sqrt gh, (hu, hv)/h, (hu^2, hv^2)/h
     template <int IXY> __host__ __device__ static constexpr int wp(int mw, int m)
@@ -324,12 +325,19 @@ struct WaveShallowFWave {
 // clawpack46_rpt2_euler4.f:56-94.  The waves stay in shared memory between the phases.
 // ---------------------------------------------------------------------------
 struct WaveEulerExact {
-    static constexpr int MEQN = 4, MWAVES = 3, MAUX = 0, NPRE = 8, NW = 12, NFL = 5;
+    static constexpr int MEQN = 4, MWAVES = 3, MAUX = 0, NPRE = 8, NW = 12, NFL = 5, NCONST = 7;
     static constexpr bool FWAVE = false, DEPTH = false, EXACT = true, SOURCE = false;
     static constexpr int NEWTON_FAILED = RPEulerExact::NEWTON_FAILED;
     // velocities, pressure, sound speed, sqrt rho, (rho u, rho v, E + p)/sqrt rho
     enum { P_U1 = 0, P_U2 = 1, P_P = 2, P_A = 3, P_RS = 4, P_N1 = 5, P_N2 = 6, P_H = 7 };
     template <int IXY> __host__ __device__ static constexpr int wp(int mw, int m) { return 4 * mw + m; }
+    // functions of gamma (Toro's G1..G7)
+    template <typename T> __device__ static void constants(T gam, T* k)
+    {
+        k[0] = (gam - T(1)) / (T(2) * gam); k[1] = (gam + T(1)) / (T(2) * gam);
+        k[2] = T(2) * gam / (gam - T(1)); k[3] = T(2) / (gam - T(1)); k[4] = T(2) / (gam + T(1));
+        k[5] = (gam - T(1)) / (gam + T(1)); k[6] = (gam - T(1)) / T(2);
+    }
     __device__ static void pre(const double* q, const WavePar<double>& P, double* c)
     {
         const double gamma1 = P.gamma - 1.0, r = q[0];
@@ -402,9 +410,7 @@ struct WaveEulerExact {
         constexpr int UN = IXY == 1 ? P_U1 : P_U2, UT = IXY == 1 ? P_U2 : P_U1;
         const double gam = P.gamma, gamma1 = gam - 1.0;
         roe<IXY>(qL, qR, cL, cR, gamma1, st.ex);
-        const double g1 = (gam - 1.0) / (2.0 * gam), g2 = (gam + 1.0) / (2.0 * gam);
-        const double g3 = 2.0 * gam / (gam - 1.0), g4 = 2.0 / (gam - 1.0), g5 = 2.0 / (gam + 1.0);
-        const double g6 = (gam - 1.0) / (gam + 1.0), g7 = (gam - 1.0) / 2.0;
+        const double g1 = P.k[0], g2 = P.k[1], g3 = P.k[2], g4 = P.k[3], g5 = P.k[4], g6 = P.k[5], g7 = P.k[6];
         const double rl = qL[0], ul = cL(UN), vl = cL(UT), pl = cL(P_P), al = cL(P_A);
         const double rr = qR[0], ur = cR(UN), vr = cR(UT), pr = cR(P_P), ar = cR(P_A);
         const double du = ur - ul;
@@ -516,9 +522,7 @@ struct WaveEulerExact {
         constexpr int UN = IXY == 1 ? P_U1 : P_U2, UT = IXY == 1 ? P_U2 : P_U1;
         const float gam = (float)P.gamma, gamma1 = gam - 1.0f;
         roe<IXY>(qL, qR, cL, cR, gamma1, st.ex);
-        const float g1 = (gam - 1.0f) / (2.0f * gam), g2 = (gam + 1.0f) / (2.0f * gam);
-        const float g3 = 2.0f * gam / (gam - 1.0f), g4 = 2.0f / (gam - 1.0f), g5 = 2.0f / (gam + 1.0f);
-        const float g6 = (gam - 1.0f) / (gam + 1.0f), g7 = (gam - 1.0f) / 2.0f;
+        const float g1 = P.k[0], g2 = P.k[1], g3 = P.k[2], g4 = P.k[3], g5 = P.k[4], g6 = P.k[5], g7 = P.k[6];
         const float rl = qL[0], ul = cL(UN), vl = cL(UT), pl = cL(P_P), al = cL(P_A);
         const float rr = qR[0], ur = cR(UN), vr = cR(UT), pr = cR(P_P), ar = cR(P_A);
         int it = 0;
