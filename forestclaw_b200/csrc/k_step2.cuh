@@ -13,14 +13,12 @@
 //   the conservative q update over i,j = 1-mbc..mx+mbc-1 (clawpack46_step2_wrap.f:107-125)
 //   and the warp-shuffle CFL maximum.
 //
-// It serves the scalar advection apps and application solvers; the flux-form systems
-// (shallow water, Euler) have their own kernel, k_wave.cuh.
+// It runs application solvers (include/fc2d_b200_user.cuh); the package's own have kernels of
+// their own, k_wave.cuh (shallow water, Euler) and k_adv.cuh (advection).
 //
-// TW is the arithmetic type of the waves, speeds, limiter, second-order
-// correction and transverse splitting.  TW = double is the FP64 path (built
-// without FMA contraction: bitwise equal to the FP64 CPU path).  TW = float is
-// the FP32-wave path: the Godunov split, the flux arrays fm/fp/gm/gp, the q update,
-// the time-sync registers and the CFL reduction stay FP64.
+// TW is the arithmetic type of the waves, speeds, limiter, second-order correction and
+// transverse splitting; built without FMA contraction, TW = double gives the bits of the FP64
+// CPU path.
 //
 // Index conventions: padded 0-based cell (ic, jc), ic = i + mbc - 1 for the
 // Fortran index i.  Interface ic sits between cells ic-1 and ic.
@@ -49,7 +47,6 @@ struct RPHooks<RP, std::void_t<decltype(RP::USER_HOOKS)>> {
 
 template <class RP, int MX, int MY, int MBC, typename TW, int NT = 0>
 struct Step2Geom {
-    static constexpr bool F32 = std::is_same<TW, float>::value;
     static constexpr int NX = MX + 2 * MBC, NY = MY + 2 * MBC, NXY = NX * NY;
     static constexpr int MEQN = RP::MEQN, MWAVES = RP::MWAVES, MAUX = RP::MAUX, NEXTRA = RP::NEXTRA;
     static constexpr int NIX = (NY - 2) * (NX - 1);          // x-sweep interfaces
@@ -70,7 +67,7 @@ struct Step2Geom {
     static constexpr int TSZ = 4 * MEQN;
     static constexpr int AUXS = MAUX > 0 ? MAUX : 0;
     static constexpr size_t DOUBLES = (size_t)MEQN * NXY * 5 + (size_t)AUXS * NXY + 64;
-    static constexpr size_t TWS = (size_t)WSZ * NI + (size_t)TSZ * NI + (F32 ? (size_t)MEQN * NXY : 0);
+    static constexpr size_t TWS = (size_t)WSZ * NI + (size_t)TSZ * NI;
     static constexpr size_t SMEM_BYTES = DOUBLES * 8 + TWS * sizeof(TW) + NI;
     // conservation registers (fclaw2d_clawpatch_conservation.h:56-77), per patch
     static constexpr int R_FP0 = 0, R_FP1 = MY * MEQN, R_FM0 = 2 * MY * MEQN, R_FM1 = 3 * MY * MEQN;
@@ -90,7 +87,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
             const StepParams& sp, unsigned long long* __restrict__ cfl_bits)
 {
     using G = Step2Geom<RP, MX, MY, MBC, TW, NT>;
-    constexpr bool F32 = G::F32, REG = G::REG;
+    constexpr bool REG = G::REG;
     constexpr int NX = G::NX, NY = G::NY, NXY = G::NXY, MEQN = G::MEQN, MWAVES = G::MWAVES;
     constexpr int MAUX = G::MAUX, NEXTRA = G::NEXTRA, NI = G::NI, WSZ = G::WSZ;
     constexpr int MA = MAUX > 0 ? MAUX : 1;
@@ -114,8 +111,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     double* red = As + G::AUXS * NXY;               // 64 doubles for reductions
     TW* W = reinterpret_cast<TW*>(red + 64);        // [WSZ][NI]  (SoA)
     TW* Tt = W + (size_t)WSZ * NI;                  // [TSZ][NI]
-    TW* Qf = Tt + (size_t)G::TSZ * NI;              // [MEQN][NY][NX] q in TW (FP32-wave path)
-    unsigned char* tflag = reinterpret_cast<unsigned char*>(Qf + (F32 ? MEQN * NXY : 0));
+    unsigned char* tflag = reinterpret_cast<unsigned char*>(Tt + (size_t)G::TSZ * NI);
 
     const int tid = threadIdx.x;
     const PatchDesc pd = desc[p];
@@ -133,7 +129,6 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
         double v = qg[k];
         if (!isfinite(v)) bad |= STATUS_NONFINITE;
         Qs[k] = v;
-        if (F32) Qf[k] = (TW)v;
         if (save) qlast[(size_t)p * MEQN * NXY + k] = v;
         FMs[k] = 0.0; FPs[k] = 0.0; GMs[k] = 0.0; GPs[k] = 0.0;
     }
@@ -177,15 +172,11 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     auto dtdy1d_y = [&](int ic, int jc) -> TW {
         return mcapa > 0 ? (TW)(dtdy / As[(mcapa - 1) * NXY + jc * NX + ic]) : (TW)dtdy;
     };
-    auto qload = [&](int m, int c) -> TW {
-        if constexpr (F32) { return Qf[m * NXY + c]; }
-        else { return (TW)Qs[m * NXY + c]; }
-    };
+    auto qload = [&](int m, int c) -> TW { return (TW)Qs[m * NXY + c]; };
     const TW gravw = (TW)sp.grav, drytolw = (TW)sp.dry_tolerance;
 
     double* rg = regs + (size_t)p * G::NREG;
     double cflmax = 0.0;
-    TW cflw = TW(0);
 
     struct State { TW wave[MWAVES][MEQN]; TW s[MWAVES]; TW am[MEQN]; TW ap[MEQN]; TW ex[NEXTRA]; };
 
@@ -203,12 +194,8 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
             for (int e = 0; e < NEXTRA; e++) W[(G::W_EX + e) * NI + k] = st.ex[e];
         }
         if (cfl_range) {
-            if (F32) {
-                for (int mw = 0; mw < MWAVES; mw++) cflw = dmax1(dmax1(cflw, d1 * st.s[mw]), -(d0 * st.s[mw]));
-            } else {
-                for (int mw = 0; mw < MWAVES; mw++)
-                    cflmax = dmax1(dmax1(cflmax, (double)(d1 * st.s[mw])), (double)(-(d0 * st.s[mw])));
-            }
+            for (int mw = 0; mw < MWAVES; mw++)
+                cflmax = dmax1(dmax1(cflmax, (double)(d1 * st.s[mw])), (double)(-(d0 * st.s[mw])));
         }
     };
     auto restore = [&](int k, State& st) {
@@ -230,15 +217,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
         TW cq[MEQN];
         for (int m = 0; m < MEQN; m++) { cq[m] = TW(0); faddm[m] = 0.0; faddp[m] = 0.0; }
         if (god) {
-            if constexpr (F32) {
-                double am64[MEQN], ap64[MEQN], qL[MEQN], qR[MEQN], aR[MA];
-                for (int m = 0; m < MEQN; m++) { qL[m] = Qs[m * NXY + cL]; qR[m] = Qs[m * NXY + cR]; }
-                for (int a = 0; a < MAUX; a++) aR[a] = As[a * NXY + cR];
-                RP::godunov64(ixy, qL, qR, aR, am64, ap64);
-                for (int m = 0; m < MEQN; m++) { faddp[m] = faddp[m] - ap64[m]; faddm[m] = faddm[m] + am64[m]; }
-            } else {
-                for (int m = 0; m < MEQN; m++) { faddp[m] = faddp[m] - (double)st.ap[m]; faddm[m] = faddm[m] + (double)st.am[m]; }
-            }
+            for (int m = 0; m < MEQN; m++) { faddp[m] = faddp[m] - (double)st.ap[m]; faddm[m] = faddm[m] + (double)st.am[m]; }
         }
         const bool second = FWAVE ? (sp.order1 != 1) : (sp.order1 == 2);
         if (second) {
@@ -277,14 +256,8 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
                         }
                     }
                     cq[m] = c;
-                    if (F32) {
-                        const double h = 0.5 * (double)c;
-                        faddm[m] = faddm[m] + h;
-                        faddp[m] = faddp[m] + h;
-                    } else {
-                        faddm[m] = faddm[m] + (double)(TW(0.5) * c);
-                        faddp[m] = faddp[m] + (double)(TW(0.5) * c);
-                    }
+                    faddm[m] = faddm[m] + (double)(TW(0.5) * c);
+                    faddp[m] = faddp[m] + (double)(TW(0.5) * c);
                 }
             }
         }
@@ -326,30 +299,6 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
             fl = 1;
         }
         tflag[k] = fl;
-    };
-
-    // clawpack46_fix_corners (clawpack46_step2.f:242-310): at a corner of the
-    // cubed sphere (three blocks meet, no corner neighbour) the mbc x mbc corner
-    // ghost cells take rotated copies of face ghost cells before each sweep
-    // (sweep 0: x, 1: y).  Sources are face ghost cells, never corner cells, so
-    // the copies are independent.
-    const int bcc = (pd.flags / PATCH_BCC3) & 15;
-    auto fix_corners = [&](int sweep) {
-        for (int t = tid; t < 4 * MBC * MBC * MEQN; t += NT) {
-            const int m = t / (4 * MBC * MBC), r = t % (4 * MBC * MBC);
-            const int k = r / (MBC * MBC), ibc = 1 + (r % (MBC * MBC)) / MBC, jbc = 1 + r % MBC;
-            if (!((bcc >> k) & 1)) continue;
-            const int i1 = (k & 1) ? MX + ibc : 1 - ibc, j1 = (k & 2) ? MY + jbc : 1 - jbc;
-            // int(ihat - jhat), int(ihat + jhat) with ihat = 0.5 or mx + 0.5, jhat = 0.5 or my + 0.5
-            const int ih = (k & 1) ? MX : 0, jh = (k & 2) ? MY : 0;
-            const int dmi = ih - jh, dpl = ih + jh + 1;
-            const bool use_b = (sweep == 0 && (k == 0 || k == 3)) || (sweep == 1 && (k == 1 || k == 2));
-            const int id = use_b ? j1 + dmi : -j1 + dpl, jd = use_b ? -i1 + dpl : i1 - dmi;
-            const int dst = m * NXY + (j1 + MBC - 1) * NX + (i1 + MBC - 1);
-            const int src = m * NXY + (jd + MBC - 1) * NX + (id + MBC - 1);
-            Qs[dst] = Qs[src];
-            if (F32) Qf[dst] = Qf[src];
-        }
     };
 
     // x-sweep interface k -> row jc = 1 + k / (NX-1), interface ic = 1 + k % (NX-1)
@@ -454,14 +403,12 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
 
     // =================== x-sweeps (clawpack46_step2.f:113-167) ===================
     State st;
-    if (bcc) { fix_corners(0); __syncthreads(); }
     if (REG) { if (tid < G::NIX) x1(tid, st); }
     else for (int k = tid; k < G::NIX; k += NT) x1(k, st);
     __syncthreads();
     if (REG) { if (tid < G::NIX) x2(tid, st); }
     else for (int k = tid; k < G::NIX; k += NT) { restore(k, st); x2(k, st); }
     __syncthreads();
-    if (bcc) { fix_corners(1); __syncthreads(); }
     // X3 and the y-sweep normal solves touch disjoint data: one phase
     for (int c = tid; c < NXY; c += NT) x3(c);
     // =================== y-sweeps (clawpack46_step2.f:182-236) ===================
@@ -542,17 +489,10 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
                 v = v - (dtdx * (FMs[b + c + 1] - FPs[b + c]) + dtdy * (GMs[b + c + NX] - GPs[b + c])) /
                             As[(mcapa - 1) * NXY + c];
             qg[k] = v;
-        } else if (bcc) {
-            // cells the update skips keep the step's (corner-fixed) values, as the
-            // reference fixes the corners of q in place
-            const int kx = ic >= MX + MBC ? 1 : (ic < MBC ? 0 : -1);
-            const int ky = jc >= MY + MBC ? 1 : (jc < MBC ? 0 : -1);
-            if (kx >= 0 && ky >= 0 && ((bcc >> (kx + 2 * ky)) & 1)) qg[k] = Qs[k];
         }
     }
 
     // ---- CFL maximum: warp shuffles, then one atomic per CTA -----------------
-    if (F32) cflmax = (double)cflw;
     for (int off = 16; off > 0; off >>= 1) cflmax = dmax1(cflmax, __shfl_xor_sync(0xffffffffu, cflmax, off));
     if ((tid & 31) == 0) red[tid >> 5] = cflmax;
     __syncthreads();

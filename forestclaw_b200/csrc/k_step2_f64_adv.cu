@@ -1,7 +1,6 @@
 // k_step2_f64_adv.cu -- FP64 instantiations (built with -fmad=false: bitwise equal to the FP64 CPU path)
-// of the fused update for scalar advection (plane and manifold): the patch-to-CTA variants of each patch size
-// (one CTA per patch, then the persistent forms).
-#include "k_step2_variant.cuh"
+// of the fused update for scalar advection (plane and manifold; k_adv.cuh), per patch size.
+#include "k_adv.cuh"
 #include "fc2d_b200.h"
 
 namespace fcb {
@@ -9,33 +8,23 @@ namespace fcb {
 const Step2Variant* step2_table_f64_adv(int* n)
 {
     static const Step2Variant table[] = {
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 32, false, 512, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 32, false, 256, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 32, false, 256, 4, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 32, false, 1024, 1, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 16, false, 416, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 16, false, 352, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 16, false, 256, 3, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 8, false, 160, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 8, false, 128, 4, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 8, false, 64, 8, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 32, false, 512, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 32, false, 256, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 32, false, 256, 4, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 32, false, 1024, 1, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 16, false, 416, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 16, false, 352, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 16, false, 256, 3, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 8, false, 160, 2, double),
-        FCB_STEP2_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 8, false, 128, 4, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 32, false, 512, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 32, false, 1024, 1, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 16, false, 416, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, RPAdvection, 8, false, 160, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 32, false, 512, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 32, false, 1024, 1, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 16, false, 416, 2, double),
-        FCB_STEP2_VARIANT_P(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, RPAdvectionManifold, 8, false, 160, 2, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 672, 2, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 448, 3, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 448, 2, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 672, 1, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 16, 416, 2, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 16, 416, 4, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 16, 224, 4, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 8, 160, 4, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION, AdvPlane, 8, 160, 8, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, AdvManifold, 32, 672, 2, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, AdvManifold, 32, 448, 2, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, AdvManifold, 32, 672, 1, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, AdvManifold, 16, 416, 2, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, AdvManifold, 16, 416, 3, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, AdvManifold, 16, 224, 4, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, AdvManifold, 8, 160, 4, double),
+        FCB_ADV_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_ADVECTION_MANIFOLD, AdvManifold, 8, 160, 8, double),
     };
     *n = (int)(sizeof(table) / sizeof(table[0]));
     return table;

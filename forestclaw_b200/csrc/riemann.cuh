@@ -1,18 +1,7 @@
-// riemann.cuh -- __device__ Riemann solvers of the advection apps, limiters, and the pressure
-// function of the exact Euler solver (the flux-form systems' solvers: wave_solvers.cuh).
-//
-// Each solver is a struct with compile-time sizes and two device functions that
-// act on ONE interface (the per-interface body of the reference's loop over
-// i = 2-mbc..mx+mbc), so the fused update kernel can give every interface its
-// own thread.  Arithmetic follows the cited Fortran line by line, in the same
-// evaluation order, so that with FMA contraction disabled the FP64 instantiation
-// reproduces the FP64 CPU path bit for bit.
-//
-//   rpn2(ixy, qL, qR, auxL, auxR) -> wave[mw][m], s[mw], amdq[m], apdq[m], extra
-//       qL = state of cell i-1 (qr(i-1,:)), qR = state of cell i (ql(i,:)),
-//       auxL/auxR = aux of cells i-1 / i on the sweep line (the reference passes aux2 for both).
-//   rpt2(ixy, imp, qL, qR, aux1, aux2, aux3, extra, asdq) -> bmasdq[m], bpasdq[m]
-//       aux1/2/3 = aux of cell i1 = i-2+imp on the lines below / on / above the sweep line.
+// riemann.cuh -- parts the update kernels share: limiters, the pressure function, fluxes and
+// star pressure of the exact Euler solver, and uncontracted arithmetic.  The solvers themselves
+// are in wave_solvers.cuh (shallow water, Euler) and k_adv.cuh (advection); application solvers
+// run in k_step2.cuh.
 #pragma once
 #include <cuda_runtime.h>
 #include "fcb_math.cuh"
@@ -33,78 +22,6 @@ __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-
-// ---------------------------------------------------------------------------
-// Scalar advection with edge velocities in aux(:,:,1:2).
-// applications/clawpack/advection/2d/all/clawpack46_rpn2adv.f, clawpack46_rpt2adv.f
-// ---------------------------------------------------------------------------
-struct RPAdvection {
-    static constexpr int MEQN = 1, MWAVES = 1, MAUX = 2, NEXTRA = 1;
-    // FP64 Godunov split for the FP32-wave path
-    __device__ static void godunov64(int ixy, const double* qL, const double* qR, const double* aR, double* am, double* ap)
-    {
-        const double s = aR[ixy - 1], d = qR[0] - qL[0];
-        am[0] = 0.0 + dmin1(s, 0.0) * d;
-        ap[0] = 0.0 + dmax1(s, 0.0) * d;
-    }
-    template <typename T>
-    __device__ static void rpn2(int ixy, const T* qL, const T* qR, const T* auxL, const T* auxR,
-                                T wave[MWAVES][MEQN], T s[MWAVES], T amdq[MEQN], T apdq[MEQN],
-                                T extra[NEXTRA], T grav)
-    {
-        (void)auxL; (void)grav; (void)extra;
-        T delta = qR[0] - qL[0];
-        wave[0][0] = delta;
-        s[0] = auxR[ixy - 1];                       // s(i,mw) = auxl(i,iface)
-        amdq[0] = T(0) + dmin1(s[0], T(0)) * wave[0][0];
-        apdq[0] = T(0) + dmax1(s[0], T(0)) * wave[0][0];
-    }
-    template <typename T>
-    __device__ static void rpt2(int ixy, int imp, const T* qL, const T* qR, const T* aux1, const T* aux2,
-                                const T* aux3, const T extra[NEXTRA], const T* asdq, T* bm, T* bp, T grav, T drytol)
-    {
-        (void)imp; (void)qL; (void)qR; (void)aux1; (void)extra; (void)grav; (void)drytol;
-        const int kv = 3 - ixy;
-        bm[0] = dmin1(aux2[kv - 1], T(0)) * asdq[0];
-        bp[0] = dmax1(aux3[kv - 1], T(0)) * asdq[0];
-    }
-};
-
-// ---------------------------------------------------------------------------
-// Scalar advection on a manifold: aux = (capacity kappa, x-edge normal velocity,
-// y-edge normal velocity), the edge velocities scaled by the edge length (psi
-// differences).  applications/clawpack/advection/2d/all/clawpack46_rpn2adv_manifold.f,
-// clawpack46_rpt2adv_manifold.f
-// ---------------------------------------------------------------------------
-struct RPAdvectionManifold {
-    static constexpr int MEQN = 1, MWAVES = 1, MAUX = 3, NEXTRA = 1;
-    __device__ static void godunov64(int ixy, const double* qL, const double* qR, const double* aR, double* am, double* ap)
-    {
-        const double s = aR[ixy], d = qR[0] - qL[0];
-        am[0] = dmin1(s, 0.0) * d;
-        ap[0] = dmax1(s, 0.0) * d;
-    }
-    template <typename T>
-    __device__ static void rpn2(int ixy, const T* qL, const T* qR, const T* auxL, const T* auxR,
-                                T wave[MWAVES][MEQN], T s[MWAVES], T amdq[MEQN], T apdq[MEQN],
-                                T extra[NEXTRA], T grav)
-    {
-        (void)auxL; (void)grav; (void)extra;
-        wave[0][0] = qR[0] - qL[0];                 // ql(i) - qr(i-1)
-        s[0] = auxR[ixy];                           // auxl(i, 1 + ixy)
-        amdq[0] = dmin1(s[0], T(0)) * wave[0][0];
-        apdq[0] = dmax1(s[0], T(0)) * wave[0][0];
-    }
-    template <typename T>
-    __device__ static void rpt2(int ixy, int imp, const T* qL, const T* qR, const T* aux1, const T* aux2,
-                                const T* aux3, const T extra[NEXTRA], const T* asdq, T* bm, T* bp, T grav, T drytol)
-    {
-        (void)imp; (void)qL; (void)qR; (void)aux1; (void)extra; (void)grav; (void)drytol;
-        const int iface = 3 - ixy;                  // aux(i1, iface + 1)
-        bm[0] = dmin1(aux2[iface], T(0)) * asdq[0];
-        bp[0] = dmax1(aux3[iface], T(0)) * asdq[0];
-    }
-};
 
 // ---------------------------------------------------------------------------
 // 2D Euler, exact Riemann solver (no counterpart in the reference): the pressure function,
