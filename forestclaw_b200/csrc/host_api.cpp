@@ -31,13 +31,14 @@ static double wall_ms()
 }
 
 // A variant with the method fixed at compile time (spec = its limiter) applies to the
-// second-order method with second-order transverse terms, that limiter on every one of the
-// three waves and no capacity.
+// second-order method with second-order transverse terms, that limiter on every wave (one of
+// advection, three of the systems) and the capacity in aux field 1 on a manifold, else none.
 static bool spec_applies(const Step2Variant& v, const fc2d_b200_options_t& o)
 {
     if (v.spec == 0) return true;
-    if (o.order[0] != 2 || o.order[1] != 2 || o.mcapa != 0) return false;
-    for (int w = 0; w < 3; w++)
+    const bool manifold = v.rp == FC2D_B200_RP_ADVECTION_MANIFOLD, adv = manifold || v.rp == FC2D_B200_RP_ADVECTION;
+    if (o.order[0] != 2 || o.order[1] != 2 || o.mcapa != (manifold ? 1 : 0)) return false;
+    for (int w = 0; w < (adv ? 1 : 3); w++)
         if (o.mthlim[w] != v.spec) return false;
     return true;
 }

@@ -36,9 +36,9 @@
 
 namespace fcb {
 
-// aux fields of the x- and y-face velocities; SWIRL: aux may hold psi differences to be scaled
-struct AdvPlane { static constexpr int MAUX = 2, U = 0, V = 1; };
-struct AdvManifold { static constexpr int MAUX = 3, U = 1, V = 2; };
+// aux fields of the x- and y-face velocities and (1-based, 0: none) of the capacity
+struct AdvPlane { static constexpr int MAUX = 2, U = 0, V = 1, CAPA = 0; };
+struct AdvManifold { static constexpr int MAUX = 3, U = 1, V = 2, CAPA = 1; };
 
 template <class RP, int MX, typename TW>
 struct AdvGeom {
@@ -59,12 +59,27 @@ struct AdvGeom {
                          R_GM0 = R_GP0 + 2 * MX, R_GM1 = R_GP0 + 3 * MX, NREG = R_GP0 + 4 * MX + 4 * MY + 4 * MX;
 };
 
-template <class RP, int MX, typename TW>
+// Method of a launch: LIM > 0 fixes it at compile time (second order, second-order transverse
+// terms, that limiter, and the capacity in aux field 1 of a manifold, none on the plane).
+template <int LIM, int CAPA>
+struct AdvMethod {
+    int o1, o2, l, m;
+    __device__ explicit AdvMethod(const StepParams* sp)
+        : o1(LIM ? 2 : sp->order1), o2(LIM ? 2 : sp->order2), l(LIM ? LIM : sp->mthlim[0]), m(LIM ? CAPA : sp->mcapa)
+    {
+    }
+    __device__ __forceinline__ int order1() const { return LIM ? 2 : o1; }
+    __device__ __forceinline__ int order2() const { return LIM ? 2 : o2; }
+    __device__ __forceinline__ int limiter() const { return LIM ? LIM : l; }
+    __device__ __forceinline__ int mcapa() const { return LIM ? CAPA : m; }
+};
+
+template <class RP, int MX, typename TW, int LIM>
 struct AdvPatch {
     using G = AdvGeom<RP, MX, TW>;
     static constexpr int NX = G::NX, NY = G::NY, NXY = G::NXY, MBC = G::MBC, MY = G::MY;
     unsigned char* sm;
-    int order1, order2, lim, mcapa;
+    AdvMethod<LIM, RP::CAPA> M;
     double dtdx, dtdy;
     bool plane;                  // the ratio plane serves both directions
 
@@ -89,9 +104,9 @@ struct AdvPatch {
     // dt/dx of cell c in direction IXY, with a capacity dt / (dx kappa)
     template <int IXY> __device__ __forceinline__ TW ratio(int c) const
     {
-        if (mcapa > 0) {
+        if (M.mcapa() > 0) {
             if (G::MAUX == 3 && (IXY == 1 || plane)) return R()[c];
-            return (TW)((IXY == 1 ? dtdx : dtdy) / A(mcapa - 1)[c]);
+            return (TW)((IXY == 1 ? dtdx : dtdy) / A(M.mcapa() - 1)[c]);
         }
         return (TW)(IXY == 1 ? dtdx : dtdy);
     }
@@ -101,23 +116,23 @@ struct AdvPatch {
     template <int IXY>
     __device__ __forceinline__ void face(int c, int pos, TW& cfl) const
     {
-        constexpr int step = IXY == 1 ? 1 : NX, M = MX;
+        constexpr int step = IXY == 1 ? 1 : NX;
         const double sd = vel<IXY>(c);
         const TW s = (TW)sd;
         const TW* q = Qt();
         TW d = q[c] - q[c - step];
         F<IXY>()[c] = G::F32 ? sd * (Q()[c] - Q()[c - step]) : (double)(s * d);
-        const bool inner = pos >= MBC && pos <= M + MBC;
+        const bool inner = pos >= MBC && pos <= MX + MBC;
         const TW rl = ratio<IXY>(c - step), rr = ratio<IXY>(c);
         if (inner) cfl = dmax1(dmax1(cfl, rr * s), -(rl * s));
         TW cq = TW(0);
-        if (order1 == 2) {
-            if (inner && lim != 0) {
+        if (M.order1() == 2) {
+            if (inner && M.limiter() != 0) {
                 // inline limiter (clawpack46_inlinelimiter.f:267-343), upwind difference
                 const int cu = s > TW(0) ? c - step : c + step;
                 const TW du = q[cu] - q[cu - step];
                 const TW wnorm2 = d * d;
-                if (wnorm2 != TW(0)) d = limiter_phi<TW>(lim, (du * d) / wnorm2) * d;
+                if (wnorm2 != TW(0)) d = limiter_phi<TW>(M.limiter(), (du * d) / wnorm2) * d;
             }
             const TW sa = fabs(s), dave = TW(0.5) * (rl + rr);
             cq = mul_rn(mul_rn(sa, sub_rn(TW(1), mul_rn(sa, dave))), d);
@@ -128,12 +143,12 @@ struct AdvPatch {
     template <int IXY> __device__ __forceinline__ TW minus(int c, int pos) const
     {
         const TW a = vel<IXY>(c) < 0.0 ? (TW)F<IXY>()[c] : TW(0);
-        return order1 > 1 && order2 == 2 && pos <= MX + 2 * MBC - 2 ? a + C<IXY>()[c] : a;
+        return M.order1() > 1 && M.order2() == 2 && pos <= MX + 2 * MBC - 2 ? a + C<IXY>()[c] : a;
     }
     template <int IXY> __device__ __forceinline__ TW plus(int c) const
     {
         const TW a = vel<IXY>(c) > 0.0 ? (TW)F<IXY>()[c] : TW(0);
-        return order1 > 1 && order2 == 2 ? a - C<IXY>()[c] : a;
+        return M.order1() > 1 && M.order2() == 2 ? a - C<IXY>()[c] : a;
     }
     // Fluxes fm, fp of the face left of (IXY 1) or below (IXY 2) cell c: own terms and the
     // transverse terms of the crossing sweep from the upwind line, whose cell there is cu.
@@ -147,7 +162,7 @@ struct AdvPatch {
         const bool god = pos <= N - 2;
         fm = (god && s < 0.0 ? a : 0.0) + h;
         fp = (god && s > 0.0 ? 0.0 - a : 0.0) + h;
-        if (order2 > 0 && (s > 0.0 ? pos - 1 >= 1 : s < 0.0 && god)) {
+        if (M.order2() > 0 && (s > 0.0 ? pos - 1 >= 1 : s < 0.0 && god)) {
             const int cu = s > 0.0 ? c - step : c;
             const TW sv = (TW)s, r = TW(0.5) * ratio<3 - IXY>(cu);
             double v = 0.0 - (double)(r * (sv * minus<3 - IXY>(cu + cross, npos + 1)));
@@ -158,7 +173,7 @@ struct AdvPatch {
     }
 };
 
-template <class RP, int MX, int NT, int MINB, typename TW>
+template <class RP, int MX, int NT, int MINB, typename TW, int LIM>
 __global__ void __launch_bounds__(NT, MINB)
 adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __restrict__ aux,
            double* __restrict__ regs, const PatchDesc* __restrict__ desc, int p0,
@@ -188,7 +203,7 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
     const double dx = pd->dx, dy = pd->dy;
     const double dt = sp->inst_dt ? sp->dt * sp->inst_dt[pd->inst] : sp->dt;
     const int bcc = (pd->flags / PATCH_BCC3) & 15;
-    const AdvPatch<RP, MX, TW> X{sm, sp->order1, sp->order2, sp->mthlim[0], sp->mcapa, dt / dx, dt / dy, dx == dy};
+    const AdvPatch<RP, MX, TW, LIM> X{sm, AdvMethod<LIM, RP::CAPA>(sp), dt / dx, dt / dy, dx == dy};
     double* Q = X.Q();
     __syncthreads();                                        // the barrier word is initialised
     const bool arrived = mbar_wait(bar, 0u, BULK_WAIT_LIMIT);
@@ -211,7 +226,7 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
             X.A(0)[c] = vty * X.A(0)[c];
             X.A(1)[c] = -(vtx * X.A(1)[c]);
         }
-        if (G::MAUX == 3 && X.mcapa > 0) X.R()[c] = (TW)(X.dtdx / X.A(X.mcapa - 1)[c]);
+        if (G::MAUX == 3 && X.M.mcapa() > 0) X.R()[c] = (TW)(X.dtdx / X.A(X.M.mcapa() - 1)[c]);
     }
     if (bad && sp->status) atomicOr(sp->status, bad);
     if (__syncthreads_or(!arrived)) {
@@ -309,8 +324,8 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
                 if (jc >= 1) X.template flux<2>(c, jc, ic, none, gb);
             }
             double v = Q[c];
-            if (X.mcapa == 0) v = v - X.dtdx * (fr - fl) - X.dtdy * (gt - gb);
-            else v = v - (X.dtdx * (fr - fl) + X.dtdy * (gt - gb)) / X.A(X.mcapa - 1)[c];
+            if (X.M.mcapa() == 0) v = v - X.dtdx * (fr - fl) - X.dtdy * (gt - gb);
+            else v = v - (X.dtdx * (fr - fl) + X.dtdy * (gt - gb)) / X.A(X.M.mcapa() - 1)[c];
             qg[c] = v;
         } else if (bcc) {
             // cells the update skips keep the step's (corner-fixed) values, as the
@@ -336,14 +351,14 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
     }
 }
 
-template <class RP, int MX, int NT, int MINB, typename TW>
+template <class RP, int MX, int NT, int MINB, typename TW, int LIM>
 cudaError_t run_adv_variant(double* q, double* qlast, const double* aux, double* regs, const PatchDesc* desc, int p0,
                             int npatch, const StepParams* sp, const LevelGroup& lg, unsigned long long* cfl_bits,
                             cudaStream_t st)
 {
     using G = AdvGeom<RP, MX, TW>;
     static bool attr_set = false;
-    auto kern = adv_kernel<RP, MX, NT, MINB, TW>;
+    auto kern = adv_kernel<RP, MX, NT, MINB, TW, LIM>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::BYTES);
         if (e != cudaSuccess) return e;
@@ -353,9 +368,10 @@ cudaError_t run_adv_variant(double* q, double* qlast, const double* aux, double*
     return launch_k(kern, npatch, NT, G::BYTES, st, q, qlast, aux, regs, desc, p0, sp, lg, cfl_bits);
 }
 
-// One table entry: precision, solver id, square patch size MXV (mbc 2), threads, CTAs per SM.
-#define FCB_ADV_VARIANT(PREC, RPID, RPT, MXV, NT, MINB, TW)                                             \
+// One table entry: precision, solver id, square patch size MXV (mbc 2), threads, CTAs per SM,
+// limiter fixed at compile time (0: any method).
+#define FCB_ADV_VARIANT(PREC, RPID, RPT, MXV, NT, MINB, TW, LIM)                                             \
     Step2Variant{PREC, RPID, MXV, MXV, 2, NT, MINB, 0, (int)AdvGeom<RPT, MXV, TW>::BYTES, 0,            \
-                 &run_adv_variant<RPT, MXV, NT, MINB, TW>, 0}
+                 &run_adv_variant<RPT, MXV, NT, MINB, TW, LIM>, LIM}
 
 }  // namespace fcb
