@@ -190,8 +190,8 @@ struct fc2d_b200_solver {
     bool use_mlp = false;
     // batch of independent forests (instances); empty: one forest of the options
     std::vector<fc2d_b200_instance_t> insts;
-    double* inst_dt_dev = nullptr;                 // coarse dt of each instance (device)
-    double* inst_dt_host = nullptr;                // pinned staging copy
+    double* inst_dt_dev = nullptr;                 // coarse dt of each instance (in the step block)
+    double* inst_dt_host = nullptr;                // its host copy
     int ncfl = 1;                                  // CFL maxima kept (one per instance)
     bool pending = false;                          // advance launched, not yet finished
     double pending_t = 0.0;
@@ -244,10 +244,16 @@ struct fc2d_b200_solver {
     // sync at the end of an advance applies them.
     int reg_pending[34] = {0};
     LevelRanges lr[33];
+    // What an advance sends and gets back, each in one copy.  The step block, on the device and
+    // page-locked: status word, CFL maxima (both zero on the host), the instances' dt, the
+    // parameters of every update launch; result_host: status word and CFL maxima after the step.
+    static constexpr size_t BLK_CFL = 16, BLK_DT = BLK_CFL + 8 * FC2D_B200_MAX_INSTANCES,
+                            BLK_PARAMS = BLK_DT + 8 * FC2D_B200_MAX_INSTANCES;
+    char* block_dev = nullptr;
+    char* block_host = nullptr;
+    char* result_host = nullptr;
     unsigned long long* cfl_dev = nullptr;
-    unsigned long long* cfl_host = nullptr;
     unsigned int* status_dev = nullptr;            // device status word (STATUS_* bits)
-    unsigned int* status_host = nullptr;           // pinned copy read with the CFL
     double* mass_dev = nullptr;
     int mass_cap = 0;
     // one forest partitioned over ranks (fc2d_b200_set_partition); null: one rank
@@ -288,8 +294,10 @@ struct fc2d_b200_solver {
     // the most recent advance: host time building its schedule (the first traversal),
     // and the span of its work on the stream (events before the first copy and after
     // the last launch), fc2d_b200_last_step_timing
-    cudaEvent_t step_ev[2] = {nullptr, nullptr};
-    double step_host_ms = 0, step_device_ms = 0;
+    // (two pairs in turn: the last finished advance keeps its events while the next runs)
+    cudaEvent_t step_ev[2][2] = {};
+    int step_pair = 0, step_done = -1;             // pair of the next advance, of the last finished one
+    double step_host_ms = 0;
     // per-launch update parameters in device memory (filled each advance)
     static constexpr int PCAP = 1 << 14;
     StepParams* params_dev = nullptr;
@@ -1036,14 +1044,22 @@ extern "C" int fc2d_b200_create(const fc2d_b200_options_t* opt, fc2d_b200_solver
         app_sphere_flow(s->o, s->flow.axis, &s->flow.omega);
     }
     CK(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
-    CK(cudaMalloc(&s->cfl_dev, sizeof(unsigned long long) * FC2D_B200_MAX_INSTANCES));
-    CK(cudaMallocHost(&s->cfl_host, sizeof(unsigned long long) * FC2D_B200_MAX_INSTANCES));
-    CK(cudaMalloc(&s->status_dev, sizeof(unsigned int)));
-    CK(cudaMemset(s->status_dev, 0, sizeof(unsigned int)));
-    CK(cudaMallocHost(&s->status_host, sizeof(unsigned int)));
-    CK(cudaMalloc(&s->inst_dt_dev, sizeof(double) * FC2D_B200_MAX_INSTANCES));
-    CK(cudaMallocHost(&s->inst_dt_host, sizeof(double) * FC2D_B200_MAX_INSTANCES));
-    CK(cudaMalloc(&s->params_dev, sizeof(StepParams) * fc2d_b200_solver::PCAP));
+    {
+        using S = fc2d_b200_solver;
+        static_assert(S::BLK_PARAMS % alignof(StepParams) == 0, "parameter blocks follow aligned");
+        const size_t bytes = S::BLK_PARAMS + sizeof(StepParams) * S::PCAP;
+        CK(cudaMalloc(&s->block_dev, bytes));
+        CK(cudaMemset(s->block_dev, 0, S::BLK_PARAMS));
+        CK(cudaMallocHost(&s->block_host, bytes));
+        std::memset(s->block_host, 0, S::BLK_PARAMS);
+        CK(cudaMallocHost(&s->result_host, S::BLK_DT));
+        s->status_dev = reinterpret_cast<unsigned int*>(s->block_dev);
+        s->cfl_dev = reinterpret_cast<unsigned long long*>(s->block_dev + S::BLK_CFL);
+        s->inst_dt_dev = reinterpret_cast<double*>(s->block_dev + S::BLK_DT);
+        s->inst_dt_host = reinterpret_cast<double*>(s->block_host + S::BLK_DT);
+        s->params_dev = reinterpret_cast<StepParams*>(s->block_dev + S::BLK_PARAMS);
+        s->params_host = reinterpret_cast<StepParams*>(s->block_host + S::BLK_PARAMS);
+    }
     {
         double bc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         s->has_inflow = app_inflow_state(s->o, bc);
@@ -1052,7 +1068,6 @@ extern "C" int fc2d_b200_create(const fc2d_b200_options_t* opt, fc2d_b200_solver
         CK(cudaMalloc(&s->newton_hist, 32 * sizeof(unsigned long long)));
         CK(cudaMemset(s->newton_hist, 0, 32 * sizeof(unsigned long long)));
     }
-    CK(cudaMallocHost(&s->params_host, sizeof(StepParams) * fc2d_b200_solver::PCAP));
     {   // set the kernel's shared-memory attribute outside any stream capture
         s->vars = step2_variants(o, o.rp);
         s->var = 0;
@@ -1074,14 +1089,13 @@ extern "C" int fc2d_b200_destroy(fc2d_b200_solver_t* s)
     cudaStreamSynchronize(s->st);
     for (auto e : s->ev_pool) cudaEventDestroy(e);
     for (auto e : s->user_ev) cudaEventDestroy(e);
-    for (auto e : s->step_ev) if (e) cudaEventDestroy(e);
+    for (auto& pair : s->step_ev)
+        for (auto e : pair) if (e) cudaEventDestroy(e);
     cudaFree(s->q); cudaFree(s->qlast); if (s->qinterp) cudaFree(s->qinterp);
     if (s->aux) cudaFree(s->aux); cudaFree(s->regs); cudaFree(s->desc);
     free_spare(s);
-    cudaFree(s->cfl_dev); cudaFreeHost(s->cfl_host); cudaFree(s->inst_dt_dev); cudaFreeHost(s->inst_dt_host);
-    cudaFree(s->status_dev); cudaFreeHost(s->status_host);
     release_graph(s);
-    cudaFree(s->params_dev); cudaFreeHost(s->params_host);
+    cudaFree(s->block_dev); cudaFreeHost(s->block_host); cudaFreeHost(s->result_host);
     if (s->mass_dev) cudaFree(s->mass_dev);
     if (s->qsave) cudaFree(s->qsave);
     if (s->ss_stage) cudaFreeHost(s->ss_stage);
@@ -1344,9 +1358,14 @@ extern "C" int fc2d_b200_get_registers(fc2d_b200_solver_t* s, double* r)
 
 static int begin_cfl(fc2d_b200_solver* s)
 {
-    CK(cudaMemsetAsync(s->cfl_dev, 0, sizeof(unsigned long long) * s->ncfl, s->st));
-    CK(cudaMemsetAsync(s->status_dev, 0, sizeof(unsigned int), s->st));
+    CK(cudaMemsetAsync(s->block_dev, 0, fc2d_b200_solver::BLK_CFL + 8 * (size_t)s->ncfl, s->st));
     return 0;
+}
+// The status word and CFL maxima of the work on the stream, to result_host.
+static cudaError_t fetch_result(fc2d_b200_solver* s)
+{
+    return cudaMemcpyAsync(s->result_host, s->block_dev, fc2d_b200_solver::BLK_CFL + 8 * (size_t)s->ncfl,
+                           cudaMemcpyDeviceToHost, s->st);
 }
 
 // The kernels' failure reports (device status word) as an error message, or "".
@@ -1361,17 +1380,18 @@ static std::string status_message(unsigned st)
     return m;
 }
 
-// Level CFL maximum (over all instances); per instance into cfl_inst if given.
+// Level CFL maximum (over all instances) once the fetched result has arrived; per instance
+// into cfl_inst if given.
 static int end_cfl(fc2d_b200_solver* s, double* cfl, double* cfl_inst = nullptr)
 {
-    CK(cudaMemcpyAsync(s->cfl_host, s->cfl_dev, sizeof(unsigned long long) * s->ncfl, cudaMemcpyDeviceToHost, s->st));
-    CK(cudaMemcpyAsync(s->status_host, s->status_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, s->st));
     CK(cudaStreamSynchronize(s->st));
-    unsigned status = *s->status_host;
+    unsigned status;
+    std::memcpy(&status, s->result_host, sizeof(status));
+    const unsigned long long* bits = reinterpret_cast<const unsigned long long*>(s->result_host + fc2d_b200_solver::BLK_CFL);
     double v = 0.0;
     bool bad = false;
     for (int i = 0; i < s->ncfl; i++) {
-        const double c = bits_to_double(s->cfl_host[i]);
+        const double c = bits_to_double(bits[i]);
         if (!(c == c)) bad = true;
         if (c > v) v = c;
         if (cfl_inst) cfl_inst[i] = c;
@@ -1408,6 +1428,7 @@ extern "C" int fc2d_b200_level_update(fc2d_b200_solver_t* s, int level, double t
     if (rc) return rc;
     rc = flush_updates(s);
     if (rc) return rc;
+    CK(fetch_result(s));
     return end_cfl(s, cfl);
 }
 
@@ -1585,23 +1606,30 @@ static int advance_launch(fc2d_b200_solver_t* s, double t, double dt)
     int rc = traverse_advance(s, t, dt);
     if (rc) { s->emit = true; return rc; }
     s->step_host_ms = wall_ms() - h0;
-    if (!s->step_ev[0]) {
-        CK(cudaEventCreate(&s->step_ev[0]));
-        CK(cudaEventCreate(&s->step_ev[1]));
+    cudaEvent_t* ev = s->step_ev[s->step_pair];
+    if (!ev[0]) {
+        CK(cudaEventCreate(&ev[0]));
+        CK(cudaEventCreate(&ev[1]));
     }
-    CK(cudaEventRecord(s->step_ev[0], s->st));
-    ProgrammaticScope pscope(s->programmatic);
+    CK(cudaEventRecord(ev[0], s->st));
     const int nupd = s->n_upd;
-    rc = begin_cfl(s);
-    if (rc) return rc;
-    if (nupd) CK(cudaMemcpyAsync(s->params_dev, s->params_host, sizeof(StepParams) * nupd, cudaMemcpyHostToDevice, s->st));
+    // the step block up, the launches, the result down
+    auto issue = [&](bool captured) -> int {
+        CK(cudaMemcpyAsync(s->block_dev, s->block_host, fc2d_b200_solver::BLK_PARAMS + sizeof(StepParams) * nupd,
+                           cudaMemcpyHostToDevice, s->st));
+        ProgrammaticScope pscope(s->programmatic, captured);
+        int r = traverse_advance(s, t, dt);
+        if (r) return r;
+        CK(fetch_result(s));
+        return 0;
+    };
     // pass 2: the launches, captured once per forest into a CUDA graph and replayed
     s->emit = true; s->fill = false;
     if (s->use_graphs && !s->timing) {
         if (s->graph_stale || !s->graph_exec || s->graph_nupd != nupd) {
             cudaGraph_t g = nullptr;
             CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
-            rc = traverse_advance(s, t, dt);
+            rc = issue(true);
             cudaError_t ec = cudaStreamEndCapture(s->st, &g);
             if (rc) { if (g) cudaGraphDestroy(g); s->fill = true; return rc; }
             if (ec != cudaSuccess) { s->fill = true; return fail(FC2D_B200_ECUDA, std::string("graph capture: ") + cudaGetErrorString(ec)); }
@@ -1629,12 +1657,12 @@ static int advance_launch(fc2d_b200_solver_t* s, double t, double dt)
         }
         CK(cudaGraphLaunch(s->graph_exec, s->st));
     } else {
-        rc = traverse_advance(s, t, dt);
+        rc = issue(false);
     }
     s->fill = true;
     if (rc) return rc;
     CK(cudaGetLastError());
-    CK(cudaEventRecord(s->step_ev[1], s->st));
+    CK(cudaEventRecord(ev[1], s->st));
     s->pending_t = t + dt;
     s->pending = true;
     return 0;
@@ -1647,11 +1675,8 @@ static int advance_finish(fc2d_b200_solver_t* s, double* maxcfl, double* cfl_ins
     if (!s->pending) return fail(FC2D_B200_ESTATE, "no advance in flight");
     s->pending = false;
     int rc = end_cfl(s, maxcfl, cfl_inst);
-    {
-        float m = 0;
-        if (s->step_ev[0] && cudaEventElapsedTime(&m, s->step_ev[0], s->step_ev[1]) == cudaSuccess) s->step_device_ms = m;
-        else { (void)cudaGetLastError(); s->step_device_ms = 0; }
-    }
+    s->step_done = s->step_pair;
+    s->step_pair ^= 1;
     if (s->timing) {
         double ms = 0, bytes = 0;
         for (auto& pr : s->upd_launch_bytes) {
@@ -1943,8 +1968,7 @@ extern "C" int fc2d_b200_restore_step(fc2d_b200_solver_t* s)
     CK(cudaMemcpyAsync(s->q, s->qsave, n * sizeof(double), cudaMemcpyDeviceToDevice, s->st));
     // the ghost cells are back to their saved values, physical ones included
     std::memcpy(s->phys_ok, s->phys_ok_save, sizeof(s->phys_ok));
-    CK(cudaStreamSynchronize(s->st));
-    return 0;
+    return 0;                                          // in stream order: no wait
 }
 
 // outstyle_1 (src/fclaw2d_run.c:113-265) with reduce_cfl (one process: the global
@@ -2182,7 +2206,15 @@ extern "C" int fc2d_b200_last_step_timing(const fc2d_b200_solver_t* s, double* h
 {
     if (!s) return fail(FC2D_B200_EINVAL, "null solver");
     if (host_ms) *host_ms = s->step_host_ms;
-    if (device_ms) *device_ms = s->step_device_ms;
+    if (device_ms) {
+        DeviceScope dev_scope_(s);
+        float m = 0;
+        if (s->step_done >= 0 && cudaEventElapsedTime(&m, s->step_ev[s->step_done][0], s->step_ev[s->step_done][1]) != cudaSuccess) {
+            (void)cudaGetLastError();
+            m = 0;
+        }
+        *device_ms = m;
+    }
     return 0;
 }
 
@@ -2663,8 +2695,7 @@ extern "C" int fc2d_b200_advance_instances_begin(fc2d_b200_solver_t* s, const do
     const int n = (int)s->insts.size();
     for (int i = 0; i < n; i++)
         if (!(dt[i] > 0.0)) return fail(FC2D_B200_EINVAL, "instance time steps must be positive");
-    std::memcpy(s->inst_dt_host, dt, sizeof(double) * n);
-    CK(cudaMemcpyAsync(s->inst_dt_dev, s->inst_dt_host, sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
+    std::memcpy(s->inst_dt_host, dt, sizeof(double) * n);      // goes up with the step block
     // the level time steps 2^-l of a unit coarse step scale each instance's own dt
     return advance_launch(s, 0.0, 1.0);
 }

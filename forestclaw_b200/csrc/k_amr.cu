@@ -19,9 +19,17 @@
 
 namespace fcb {
 
-static thread_local bool tl_programmatic = false;
-void set_programmatic_launch(bool on) { tl_programmatic = on; }
-bool programmatic_launch() { return tl_programmatic; }
+static thread_local bool tl_programmatic = false, tl_after_copy = false;
+void set_programmatic_launch(bool on, bool after_copy)
+{
+    tl_programmatic = on;
+    tl_after_copy = after_copy;
+}
+bool programmatic_launch()
+{
+    if (tl_after_copy) { tl_after_copy = false; return false; }
+    return tl_programmatic;
+}
 
 static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 

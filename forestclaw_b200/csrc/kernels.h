@@ -7,14 +7,14 @@
 
 namespace fcb {
 
-// Programmatic dependent launch of the advance's kernels (fcb_launch.cuh): set
-// for the calling thread while a ProgrammaticScope lives.
-void set_programmatic_launch(bool on);
-bool programmatic_launch();
+// Programmatic dependent launch of the advance's kernels (fcb_launch.cuh): on for the
+// calling thread while a ProgrammaticScope lives.  after_copy: the scope's first kernel
+// follows a copy, not a kernel, and is launched plainly.
+void set_programmatic_launch(bool on, bool after_copy);
+bool programmatic_launch();          // for the next launch
 struct ProgrammaticScope {
-    bool prev;
-    explicit ProgrammaticScope(bool on) : prev(programmatic_launch()) { set_programmatic_launch(on); }
-    ~ProgrammaticScope() { set_programmatic_launch(prev); }
+    ProgrammaticScope(bool on, bool after_copy) { set_programmatic_launch(on, after_copy); }
+    ~ProgrammaticScope() { set_programmatic_launch(false, false); }
 };
 
 struct Dims {
