@@ -233,7 +233,7 @@ struct fc2d_b200_solver {
     DevView<InterpEnt> t_interp;
     DevView<PhysEnt> t_phys;
     DevView<int> t_ti;
-    DevView<SyncOp> t_sync;
+    DevView<int> t_sync;
     Tables tables;                                 // host copy of the gather tables (buffers reused)
     TableWork table_work;
     std::vector<unsigned char> interp_written;     // interpolation-chain scratch, all zero between uses
@@ -455,7 +455,7 @@ static int upload_desc_and_tables(fc2d_b200_solver* s)
         filter(T.ti, T.ti_off, [&](int p) { return fill[p] != 0; });
         for (int i = 0; i < f.np(); i++)          // the corrections of owned patches only
             if (own[i] != me)
-                for (int k = 0; k < SYNC_SLOTS; k++) T.sync[(size_t)i * SYNC_SLOTS + k].kind = SYNC_NONE;
+                for (int k = 0; k < SYNC_SLOTS; k++) T.sync[(size_t)i * SYNC_SLOTS + k] = -1;
         // halo slot lists (send, then receive), uploaded once per forest
         std::vector<int> slots;
         for (const auto& v : P.plan.send) slots.insert(slots.end(), v.begin(), v.end());

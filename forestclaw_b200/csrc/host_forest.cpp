@@ -781,7 +781,7 @@ bool build_tables(const Forest& f, const int mthbc[4], bool inflow, Tables& out,
         return true;
     };
     // ---- the tables of each patch: region ops, physical BCs, time-interpolation list and
-    // time-sync ops, in chunks of up to 64 patches of one level (one task each) ----
+    // time-sync sources, in chunks of up to 64 patches of one level (one task each) ----
     struct PChunk { int l, a, b; };
     std::vector<PChunk> pch;
     for (int l = 0; l < nlev; l++)
@@ -834,33 +834,21 @@ bool build_tables(const Forest& f, const int mthbc[4], bool inflow, Tables& out,
         }
         // ---- time interpolation patches ----
         for (int ip = a0; ip < a1; ip++) if (f.p[ip].has_fine_nbr) w.ti[c].push_back(ip);
-        // ---- time sync ops ----
-        // fclaw2d_time_sync applies the same-size corrections of every synced level,
-        // then the fine-to-coarse ones (src/fclaw2d_time_sync.c:118-202); each
-        // correction adds to cells of its own patch p only and reads registers no
-        // correction writes, so per patch the samesize ops (faces 0..3) followed by
-        // the f2c ops ((face, igrid) order) give every cell its additions in the
-        // reference's order.  Levels without finer neighbours have no f2c ops, so
-        // one range of levels [a, maxlevel] covers both kinds.  A patch has at most
-        // eight ops (one samesize or two f2c per face): slots 8 p .. 8 p + 7.
+        // ---- time-sync sources: per face and half of it the neighbour whose registers
+        // correct the cells there (fclaw2d_time_sync, src/fclaw2d_time_sync.c:118-202).  Levels
+        // without finer neighbours have no half-size faces, so one range of levels
+        // [a, maxlevel] covers both kinds. ----
         for (int ip = a0; ip < a1; ip++) {
             const PatchInfo& P = f.p[ip];
-            SyncOp* slot = &out.sync[(size_t)ip * SYNC_SLOTS];
-            int nops = 0;
-            for (int fc = 0; fc < 4; fc++)
-                if (P.face_type[fc] == NB_SAME && (!f.sphere() || f.p[P.face_nbr[fc][0]].block == P.block))
-                    slot[nops++] = {ip, P.face_nbr[fc][0], fc, 0, 0, SYNC_SAMESIZE, {0, 0}};
+            int* slot = &out.sync[(size_t)ip * SYNC_SLOTS];
             for (int fc = 0; fc < 4; fc++) {
-                if (P.face_type[fc] != NB_HALF) continue;
+                slot[2 * fc] = slot[2 * fc + 1] = -1;
+                if (P.face_type[fc] != NB_SAME && P.face_type[fc] != NB_HALF) continue;
                 if (f.sphere() && f.p[P.face_nbr[fc][0]].block != P.block) continue;
-                for (int ig = 0; ig < 2; ig++) {
-                    const int fi = P.face_nbr[fc][ig];
-                    const PatchInfo& F = f.p[fi];
-                    const int noff = (fc < 2) ? (2 * P.gy - F.gy) * my : (2 * P.gx - F.gx) * mx;
-                    slot[nops++] = {ip, fi, fc, ig, noff, SYNC_F2C, {0, 0}};
-                }
+                const int half = P.face_type[fc] == NB_HALF;
+                for (int h = 0; h < 2; h++)
+                    slot[2 * fc + h] = 2 * P.face_nbr[fc][half ? h : 0] + (half ? SYNC_F2C : SYNC_SAMESIZE);
             }
-            for (; nops < SYNC_SLOTS; nops++) slot[nops] = SyncOp{0, 0, 0, 0, 0, SYNC_NONE, {0, 0}};
         }
     };
     auto patches = [&](int c) {

@@ -169,9 +169,7 @@ struct Tables {
     std::vector<InterpEnt> interp;   // interpolate2ghost(level): level is the coarse level
     std::vector<PhysEnt> phys;       // setphysical(level)
     std::vector<int> ti;             // patches with fine-grid neighbours (fclaw2d_timeinterp)
-    // time-sync corrections of patch p: sync[SYNC_SLOTS p .. SYNC_SLOTS p + 7], in the
-    // reference's order, unused slots SYNC_NONE
-    std::vector<SyncOp> sync;
+    std::vector<int> sync;           // time-sync sources, SYNC_SLOTS per patch (launch_sync)
     int copy_off[34], avg_off[34], interp_off[34], phys_off[34], ti_off[34];
 };
 

@@ -320,43 +320,24 @@ struct RegOff {
     }
 };
 
-// The corrections of a time sync, one CTA per patch of the synced levels.  A face of a
-// patch is either same-size (one samesize op) or half-size (two f2c ops,
-// igrid 0 and 1, each covering half the face), so every (face, tangential index,
-// field) has at most one correction.  The CTA files the patch's ops by face in
-// shared memory, computes every correction with one thread each (phase 1), then
-// adds them to the boundary cells with one thread per (cell, field) (phase 2):
-// a corner cell on two corrected faces takes the samesize corrections first,
-// then the f2c ones, each kind in face order -- the order of the reference's
-// additions to that cell.  Every op reads registers only, which no correction
-// writes.
+// The corrections of a time sync, one CTA per patch of the synced levels and one thread per
+// (face, field, tangential index).  A face of a patch is either same-size or half-size, so
+// every such item has at most one correction, from one neighbour (kernels.h, launch_sync):
 //   samesize: clawpack46_fort_time_sync_samesize (same orientation, sc = 1),
 //             clawpack46_time_sync.f:528-704: delta = (ef_n - ef_t) - (f_n - f_t),
 //             q += 0.5 delta / area
 //   f2c:      clawpack46_fort_time_sync_f2c (same orientation, sc = 1),
-//             clawpack46_time_sync.f:254-498: the fine pair d, d+1 (d = 1 + n_off + 2 j)
-//             of coarse cell j, skipped when outside the fine face; q += deltac / area
-// Scratch: the ops below and 4 * meqn * max(mx, my) doubles (corrections) followed
-// by as many flag bytes (sync_scratch_bytes), then the prefetched registers and cells
-// (sync_prefetch_bytes), in dynamic shared memory.
-struct SyncSmem { SyncOp op[8]; int ss[4]; int fc[4][2]; };   // op slots per face (-1: none)
-__host__ __device__ constexpr size_t sync_scratch_bytes(int mx, int my, int meqn)
-{
-    return ((size_t)4 * meqn * (mx > my ? mx : my) * (sizeof(double) + 1) + 15) / 16 * 16;
-}
-__host__ __device__ constexpr size_t sync_prefetch_bytes(int mx, int my, int meqn)
-{
-    return ((size_t)2 * 4 * meqn * (mx > my ? mx : my) + (size_t)(2 * (mx + my) - 4) * meqn) * sizeof(double);
-}
-// 8-byte asynchronous copy global -> shared (cp.async, sm_80+), and the wait for this
-// thread's copies
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
-                 "l"(gmem)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+//             clawpack46_time_sync.f:254-498: the fine pair of coarse cell j; q += deltac / area
+// A thread adds its correction to its cell; only a corner cell lies on two faces, and takes the
+// samesize corrections first, then the f2c ones, each kind in face order, as the reference adds
+// them: its corrections go through shared memory to one thread.  Every item reads registers
+// only, which no correction writes.
+//
+// Latency and issue bound (the data sits in L2).  A form that filed a patch's ops by face in
+// shared memory, prefetched registers and cells there and then computed all corrections before
+// all additions took three barriers and some 240 instructions per item; with the sources in a
+// face-indexed table the chain is source -> neighbour's registers -> add.  Radial dam levels
+// 3-7, 1960 patches: see the figures in launch_sync.
 // Patch shape and field count of the time sync: compile-time for the common shapes
 // (the index arithmetic and register offsets fold), run-time otherwise.
 template <int MX, int MEQN>
@@ -368,174 +349,86 @@ struct RunSync {
     int mx, my, mbc, meqn;
     __device__ RunSync(int mx_, int my_, int mbc_, int meqn_) : mx(mx_), my(my_), mbc(mbc_), meqn(meqn_) {}
 };
+constexpr int SYNC_MAX_MEQN = 8;
 template <class PS>
-__device__ void sync_group(const PS& P, int p, int tid, int nthr, SyncSmem& S, double* s_corr,
-                           double* __restrict__ q, const double* __restrict__ regs,
-                           const PatchDesc* __restrict__ desc, const SyncOp* __restrict__ ops, int nreg)
-{
-    const int mx = P.mx, my = P.my, mbc = P.mbc, meqn = P.meqn;
-    const int nmax = mx > my ? mx : my;
-    unsigned char* s_has = reinterpret_cast<unsigned char*>(s_corr + 4 * meqn * nmax);
-    const int nx = mx + 2 * mbc, ny = my + 2 * mbc, nxy = nx * ny;
-    const int n1 = 4 * meqn * nmax;                            // phase-1 items: (face, field, index)
-    const int ring = 2 * (mx + my) - 4;                        // interior cells on the patch boundary
-    const int n2 = ring * meqn;                                // phase-2 items: (cell, field)
-    RegOff R(mx, my, meqn);
-    const double* rt = regs + (size_t)p * nreg;
-    // phase-1 item t: face, field, index, its length, and this patch's two registers the
-    // correction reads (A: edge flux, B: fluctuation sum) at the face's side
-    auto item1 = [&](int t, int& face, int& m, int& j, int& nt, int& ra, int& rb) {
-        face = t / (meqn * nmax);
-        const int r = t % (meqn * nmax);
-        m = r / nmax;
-        j = r % nmax;
-        nt = (face < 2) ? my : mx;
-        const int o = j + m * nt;
-        ra = (face == 0 ? R.ef0 : face == 1 ? R.ef1 : face == 2 ? R.ef2 : R.ef3) + o;
-        rb = (face == 0 ? R.fp0 : face == 1 ? R.fm1 : face == 2 ? R.gp0 : R.gm1) + o;
-    };
-    // phase-2 item t: the cell's offset in q (field m plane) and its x and y faces
-    auto item2 = [&](int t, int& m, int& ic, int& jc) {
-        m = t / ring;
-        const int k = t % ring;
-        if (k < mx) { ic = mbc + k; jc = mbc; }
-        else if (k < 2 * mx) { ic = mbc + k - mx; jc = my + mbc - 1; }
-        else if (k < 2 * mx + my - 2) { ic = mbc; jc = mbc + 1 + (k - 2 * mx); }
-        else { ic = mx + mbc - 1; jc = mbc + 1 + (k - 2 * mx - (my - 2)); }
-    };
-    double* qp = q + (size_t)p * nxy * meqn;
-    // this patch's registers of every phase-1 item and boundary cells of every phase-2
-    // item, copied into shared memory (asynchronously, no registers held) while the
-    // ops arrive: neither depends on them.  Each thread reads back only its own items.
-    double* pre_r = s_corr + sync_scratch_bytes(mx, my, meqn) / sizeof(double);   // [n1][2]
-    double* pre_q = pre_r + 2 * n1;                                                // [n2]
-    for (int t = tid; t < n1; t += nthr) {
-        int face, m, j, nt, ra, rb;
-        item1(t, face, m, j, nt, ra, rb);
-        if (j < nt) { cp_async8(pre_r + 2 * t, rt + ra); cp_async8(pre_r + 2 * t + 1, rt + rb); }
-    }
-    for (int t = tid; t < n2; t += nthr) {
-        int m, ic, jc;
-        item2(t, m, ic, jc);
-        cp_async8(pre_q + t, qp + (size_t)m * nxy + jc * nx + ic);
-    }
-    const double area = desc[p].dx * desc[p].dy;
-    if (tid < 4) { S.ss[tid] = -1; S.fc[tid][0] = -1; S.fc[tid][1] = -1; }
-    if (tid < SYNC_SLOTS) S.op[tid] = ops[(size_t)p * SYNC_SLOTS + tid];
-    __syncthreads();
-    if (S.op[0].kind == SYNC_NONE) {                           // no corrections for this patch
-        cp_async_wait_all();
-        return;
-    }
-    if (tid < SYNC_SLOTS) {
-        const SyncOp& op = S.op[tid];
-        if (op.kind == SYNC_SAMESIZE) S.ss[op.face & 3] = tid;
-        else if (op.kind == SYNC_F2C) S.fc[op.face & 3][op.igrid & 1] = tid;
-    }
-    __syncthreads();
-    cp_async_wait_all();
-    // ---- phase 1: the correction of each (face, field, tangential index) ----
-    for (int t = tid; t < n1; t += nthr) {
-        int face, m, j, nt, ra, rb;
-        item1(t, face, m, j, nt, ra, rb);
-        bool has = false;
-        double corr = 0.0;
-        if (j < nt) {
-            const double rA = pre_r[2 * t], rB = pre_r[2 * t + 1];
-            if (S.ss[face] >= 0) {
-                const SyncOp& op = S.op[S.ss[face]];
-                const double* rn = regs + (size_t)op.n * nreg;
-                double delta;
-                if (face == 0) {
-                    double fp = rn[R.fp1 + j + m * my];
-                    double ef = 1 * rn[R.ef1 + j + m * my + my * meqn];
-                    delta = (ef - rA) - (fp - rB);
-                } else if (face == 1) {
-                    double fm = rn[R.fm0 + j + m * my];
-                    double ef = 1 * rn[R.ef0 + j + m * my + my * meqn];
-                    delta = (rA - ef) - (fm - rB);
-                } else if (face == 2) {
-                    double gp = rn[R.gp1 + j + m * mx];
-                    double ef = 1 * rn[R.ef3 + j + m * mx + mx * meqn];
-                    delta = (ef - rA) - (gp - rB);
-                } else {
-                    double gm = rn[R.gm0 + j + m * mx];
-                    double ef = 1 * rn[R.ef2 + j + m * mx + mx * meqn];
-                    delta = (rA - ef) - (gm - rB);
-                }
-                corr = 0.5 * delta / area;
-                has = true;
-            } else {
-                for (int ig = 0; ig < 2 && !has; ig++) {
-                    if (S.fc[face][ig] < 0) continue;
-                    const SyncOp& op = S.op[S.fc[face][ig]];
-                    const int d = 1 + op.n_off + 2 * j;        // first fine child (Fortran index)
-                    if (d < 1 || d + 1 > nt) continue;         // fc46_skip_this_grid
-                    const double* rn = regs + (size_t)op.n * nreg;
-                    const int f0 = d - 1, f1 = d;              // 0-based fine pair
-                    double deltac;
-                    if (face == 0) {
-                        double fp = rn[R.fp1 + f0 + m * my] + rn[R.fp1 + f1 + m * my];
-                        double ef = 1 * (rn[R.ef1 + f0 + m * my + my * meqn] + rn[R.ef1 + f1 + m * my + my * meqn]);
-                        deltac = (ef - rA) - (fp - rB);
-                    } else if (face == 1) {
-                        double fm = rn[R.fm0 + f0 + m * my] + rn[R.fm0 + f1 + m * my];
-                        double ef = 1 * (rn[R.ef0 + f0 + m * my + my * meqn] + rn[R.ef0 + f1 + m * my + my * meqn]);
-                        deltac = (rA - ef) - (fm - rB);
-                    } else if (face == 2) {
-                        double gp = rn[R.gp1 + f0 + m * mx] + rn[R.gp1 + f1 + m * mx];
-                        double ef = 1 * (rn[R.ef3 + f0 + m * mx + mx * meqn] + rn[R.ef3 + f1 + m * mx + mx * meqn]);
-                        deltac = (ef - rA) - (gp - rB);
-                    } else {
-                        double gm = rn[R.gm0 + f0 + m * mx] + rn[R.gm0 + f1 + m * mx];
-                        double ef = 1 * (rn[R.ef2 + f0 + m * mx + mx * meqn] + rn[R.ef2 + f1 + m * mx + mx * meqn]);
-                        deltac = (rA - ef) - (gm - rB);
-                    }
-                    corr = deltac / area;
-                    has = true;
-                }
-            }
-        }
-        s_corr[t] = corr;
-        s_has[t] = has ? 1 : 0;
-    }
-    __syncthreads();
-    // ---- phase 2: add them to the boundary cells, samesize faces first ----
-    for (int t = tid; t < n2; t += nthr) {
-        int m, ic, jc;                                         // storage indices of the cell
-        item2(t, m, ic, jc);
-        const int fx = (ic == mbc) ? 0 : (ic == mx + mbc - 1) ? 1 : -1;
-        const int fy = (jc == mbc) ? 2 : (jc == my + mbc - 1) ? 3 : -1;
-        // slots of the cell's corrections on its x and y faces, in the reference's order
-        int sl[2] = {-1, -1};
-        if (fx >= 0) sl[0] = (fx * meqn + m) * nmax + (jc - mbc);
-        if (fy >= 0) sl[1] = (fy * meqn + m) * nmax + (ic - mbc);
-        const bool xss = fx >= 0 && S.ss[fx] >= 0, yss = fy >= 0 && S.ss[fy] >= 0;
-        const int first = (!xss && yss) ? 1 : 0;               // a samesize y face goes before an f2c x face
-        double* qq = qp + (size_t)m * nxy + jc * nx + ic;
-        double v = 0.0;
-        bool touched = false;
-        for (int w = 0; w < 2; w++) {
-            const int s = sl[w ^ first];
-            if (s < 0 || !s_has[s]) continue;
-            if (!touched) { v = pre_q[t]; touched = true; }
-            v = v + s_corr[s];
-        }
-        if (touched) *qq = v;
-    }
-}
-// One CTA per patch of the synced levels: 128 threads and at most 32 registers, 16
-// CTAs per SM, so a sync of up to ~2300 patches runs in one wave.
-template <class PS>
-__global__ void __launch_bounds__(128, 16)
+__global__ void __launch_bounds__(256)
 k_sync(double* __restrict__ q, const double* __restrict__ regs, const PatchDesc* __restrict__ desc,
-       const SyncOp* __restrict__ ops, int p0, int mx, int my, int mbc, int meqn, int nreg)
+       const int* __restrict__ src, int p0, int mx_, int my_, int mbc_, int meqn_, int nreg)
 {
     grid_dependency_wait();       // programmatic launch: the previous grid's writes are visible
     grid_launch_dependents();
-    __shared__ SyncSmem S;
-    extern __shared__ double s_corr[];
-    sync_group(PS(mx, my, mbc, meqn), p0 + blockIdx.x, threadIdx.x, blockDim.x, S, s_corr, q, regs, desc, ops, nreg);
+    const PS P(mx_, my_, mbc_, meqn_);
+    const int mx = P.mx, my = P.my, mbc = P.mbc, meqn = P.meqn;
+    // corrections of the corner cells: [face][field][low or high end], and whether there is one
+    __shared__ double s_corr[4 * SYNC_MAX_MEQN * 2];
+    __shared__ unsigned char s_has[4 * SYNC_MAX_MEQN * 2];
+    const int p = p0 + blockIdx.x, nmax = mx > my ? mx : my;
+    const int nx = mx + 2 * mbc, nxy = nx * (my + 2 * mbc);
+    const RegOff R(mx, my, meqn);
+    const double* rt = regs + (size_t)p * nreg;
+    const int* sp = src + (size_t)p * SYNC_SLOTS;
+    double* qp = q + (size_t)p * nxy * meqn;
+    const double area = desc[p].dx * desc[p].dy;
+    for (int t = threadIdx.x; t < 4 * meqn * nmax; t += blockDim.x) {
+        const int j = t % nmax, fm = t / nmax, face = fm / meqn, m = fm - face * meqn;
+        const int nt = face < 2 ? my : mx;                        // cells along the face
+        if (j >= nt) continue;
+        const int half = 2 * j >= nt;
+        const int e = sp[2 * face + half];
+        const bool end = j == 0 || j == nt - 1;
+        const int o = j + m * nt, kofs = nt * meqn;
+        const bool low = (face & 1) == 0;
+        // this patch's edge flux and fluctuation sum at the face, the neighbour's (second edge
+        // flux: its cell on this side of the face), and the cell
+        const int ra = (face == 0 ? R.ef0 : face == 1 ? R.ef1 : face == 2 ? R.ef2 : R.ef3) + o;
+        const int rb = (face == 0 ? R.fp0 : face == 1 ? R.fm1 : face == 2 ? R.gp0 : R.gm1) + o;
+        const int na = (face == 0 ? R.ef1 : face == 1 ? R.ef0 : face == 2 ? R.ef3 : R.ef2) + m * nt + kofs;
+        const int nb = (face == 0 ? R.fp1 : face == 1 ? R.fm0 : face == 2 ? R.gp1 : R.gm0) + m * nt;
+        const int ic = face == 0 ? mbc : face == 1 ? mx + mbc - 1 : mbc + j;
+        const int jc = face == 2 ? mbc : face == 3 ? my + mbc - 1 : mbc + j;
+        double* qq = qp + (size_t)m * nxy + jc * nx + ic;
+        const double rA = rt[ra], rB = rt[rb];
+        const double v = end ? 0.0 : *qq;
+        double corr = 0.0;
+        if (e >= 0) {
+            const double* rn = regs + (size_t)(e >> 1) * nreg;
+            const bool f2c = e & 1;
+            double ef, fl;
+            if (f2c) {
+                const int f0 = 2 * j - half * nt;                 // fine pair f0, f0 + 1 (0-based)
+                fl = rn[nb + f0] + rn[nb + f0 + 1];
+                ef = rn[na + f0] + rn[na + f0 + 1];
+            } else {
+                fl = rn[nb + j];
+                ef = rn[na + j];
+            }
+            const double delta = (low ? ef - rA : rA - ef) - (fl - rB);
+            corr = f2c ? delta / area : 0.5 * delta / area;
+            if (!end) *qq = v + corr;
+        }
+        if (end) {
+            const int s = (face * meqn + m) * 2 + (j == 0 ? 0 : 1);
+            s_corr[s] = corr;
+            s_has[s] = e >= 0 ? 1 : 0;
+        }
+    }
+    __syncthreads();
+    // corner cell (cx, cy): x face cx at its end cy, y face 2 + cy at its end cx
+    for (int t = threadIdx.x; t < 4 * meqn; t += blockDim.x) {
+        const int m = t >> 2, cx = t & 1, cy = (t >> 1) & 1;
+        const int fx = cx, fy = 2 + cy;
+        const int sx = (fx * meqn + m) * 2 + cy, sy = (fy * meqn + m) * 2 + cx;
+        const int ex = sp[2 * fx + cy], ey = sp[2 * fy + cx];
+        // a samesize y face goes before an f2c x face
+        const bool y_first = ey >= 0 && (ey & 1) == SYNC_SAMESIZE && !(ex >= 0 && (ex & 1) == SYNC_SAMESIZE);
+        const int s0 = y_first ? sy : sx, s1 = y_first ? sx : sy;
+        if (!s_has[s0] && !s_has[s1]) continue;
+        double* qq = qp + (size_t)m * nxy + (cy ? my + mbc - 1 : mbc) * nx + (cx ? mx + mbc - 1 : mbc);
+        double v = *qq;
+        if (s_has[s0]) v = v + s_corr[s0];
+        if (s_has[s1]) v = v + s_corr[s1];
+        *qq = v;
+    }
 }
 
 // fclaw2d_time_sync's resets for levels [minlevel, maxl] (src/fclaw2d_time_sync.c:118-154):
@@ -872,8 +765,8 @@ void launch_timeinterp(const Dims& d, const double* q, const double* qlast, doub
         launch_k(k_timeinterp, nblk((long)npatch * d.nxy(), 256), 256, 0, st, q, qlast, qinterp, patches, npatch, desc,
                  d.mx, d.my, d.mbc, d.meqn, alpha);
 }
-void launch_sync(const Dims& d, double* q, const double* regs, const PatchDesc* desc, const SyncOp* ops, int p0,
-                 int np, cudaStream_t st)
+void launch_sync(const Dims& d, double* q, const double* regs, const PatchDesc* desc, const int* src, int p0, int np,
+                 cudaStream_t st)
 {
     if (np <= 0) return;
     auto kern = &k_sync<RunSync>;
@@ -882,8 +775,9 @@ void launch_sync(const Dims& d, double* q, const double* regs, const PatchDesc* 
         else if (d.mx == 16 && d.meqn == 4) kern = &k_sync<FixedSync<16, 4>>;
         else if (d.mx == 8 && d.meqn == 3) kern = &k_sync<FixedSync<8, 3>>;
     }
-    launch_k(kern, np, 128, sync_scratch_bytes(d.mx, d.my, d.meqn) + sync_prefetch_bytes(d.mx, d.my, d.meqn), st, q,
-             regs, desc, ops, p0, d.mx, d.my, d.mbc, d.meqn, d.nreg());
+    const int items = 4 * d.meqn * (d.mx > d.my ? d.mx : d.my);
+    launch_k(kern, np, items < 256 ? (items + 31) / 32 * 32 : 256, 0, st, q, regs, desc, src, p0, d.mx, d.my, d.mbc,
+             d.meqn, d.nreg());
 }
 void launch_reset_sync(const Dims& d, double* regs, const PatchDesc* desc, int p0, int np, int minlevel, int maxl,
                        cudaStream_t st)

@@ -99,17 +99,15 @@ void launch_timeinterp(const Dims& d, const double* q, const double* qlast, doub
                        int npatch, const PatchDesc* desc, const LevelAlpha& alpha, cudaStream_t st);
 
 // ---- time sync (k_amr.cu) -------------------------------------------------------
-// One time-sync correction of patch p from neighbour n across face `face`:
-// kind SYNC_SAMESIZE (clawpack46_fort_time_sync_samesize) or SYNC_F2C (coarse p,
-// fine n = child igrid of the face, n_off = first fine index offset along it).
-enum { SYNC_SAMESIZE = 0, SYNC_F2C = 1, SYNC_NONE = -1 };
-struct SyncOp { int p, n, face, igrid; int n_off; int kind; int pad[2]; };
-constexpr int SYNC_SLOTS = 8;      // ops of a patch: at most one samesize or two f2c per face
-// The corrections of a time sync over patches p0 .. p0 + np - 1: the ops of patch p are
-// ops[SYNC_SLOTS p ..] (samesize faces 0..3, then f2c ops in (face, igrid) order; the
-// rest SYNC_NONE).
-void launch_sync(const Dims& d, double* q, const double* regs, const PatchDesc* desc, const SyncOp* ops, int p0,
-                 int np, cudaStream_t st);
+// The corrections of patch p: entry SYNC_SLOTS p + 2 face + half is the source of that half of
+// the face, 2 n + kind for neighbour slot n, or -1 for no correction.  Kind SYNC_SAMESIZE
+// (clawpack46_fort_time_sync_samesize): n is the same-size neighbour, in both halves; SYNC_F2C
+// (..._f2c): n is the half-size neighbour beside that half.
+enum { SYNC_SAMESIZE = 0, SYNC_F2C = 1 };
+constexpr int SYNC_SLOTS = 8;
+// The corrections of a time sync over patches p0 .. p0 + np - 1.
+void launch_sync(const Dims& d, double* q, const double* regs, const PatchDesc* desc, const int* src, int p0, int np,
+                 cudaStream_t st);
 // All register resets of one fclaw2d_time_sync(minlevel, maxl) call in one launch
 // over the patches of levels [minlevel, maxl].
 void launch_reset_sync(const Dims& d, double* regs, const PatchDesc* desc, int p0, int np, int minlevel, int maxl,
