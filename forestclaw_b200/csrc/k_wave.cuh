@@ -191,18 +191,17 @@ struct WavePatch {
                 double a64, p64;
                 RP::fluct_mixed(st, m, flux<IXY>(m, cL), flux<IXY>(m, cR), a64, p64);
                 am[m] = (TW)a64; ap[m] = (TW)p64;
-                fp[m] = god ? 0.0 - p64 : 0.0;
+                fp[m] = god ? -p64 : 0.0;
             }
         } else {
             RP::template fluct<IXY>(st, w, s, am, ap);
 #pragma unroll
             for (int m = 0; m < MEQN; m++) {
                 if constexpr (F32) {
-                    double p64 = (double)ap[m];
+                    fp[m] = (double)(god ? -ap[m] : TW(0));
                     // zero mass flux through a wall: the interior cell's fluctuation cancels its own flux
-                    if (m == 0 && wall_lo) p64 = flux<IXY>(0, cR);
-                    if (m == 0 && wall_hi) p64 = (flux<IXY>(0, cR) - flux<IXY>(0, cL)) + flux<IXY>(0, cL);
-                    fp[m] = god ? 0.0 - p64 : 0.0;
+                    if (m == 0 && wall_lo) fp[0] = -flux<IXY>(0, cR);
+                    if (m == 0 && wall_hi) fp[0] = -((flux<IXY>(0, cR) - flux<IXY>(0, cL)) + flux<IXY>(0, cL));
                 } else {
                     fm[m] = god ? am[m] : 0.0;
                     fp[m] = god ? 0.0 - ap[m] : 0.0;
@@ -214,6 +213,9 @@ struct WavePatch {
         const TW dlo = ratio(IXY, cL);
         const TW dhi = RP::FWAVE ? dlo : ratio(IXY, cR);
         if (RP::FWAVE ? M.order1 != 1 : M.order1 == 2) {
+            TW wlim[MWAVES];
+#pragma unroll
+            for (int mw = 0; mw < MWAVES; mw++) wlim[mw] = TW(1);
             if (pos >= MBC && pos <= MX + MBC) {
                 // inline limiter (clawpack46_inlinelimiter.f:267-343): the projection of the
                 // upwind neighbour's unlimited wave
@@ -230,9 +232,13 @@ struct WavePatch {
                         dot = dot + W()[RP::template wp<IXY>(mw, m) * NI + kk] * w[mw][m];
                     }
                     if (wnorm2 == TW(0)) continue;
-                    const TW wlim = limiter_phi<TW>(ml, dot / wnorm2);
+                    const TW phi = limiter_phi<TW>(ml, dot / wnorm2);
+                    if constexpr (F32) {
+                        wlim[mw] = phi;                         // goes into the correction's factor
+                    } else {
 #pragma unroll
-                    for (int m = 0; m < MEQN; m++) w[mw][m] = wlim * w[mw][m];
+                        for (int m = 0; m < MEQN; m++) w[mw][m] = phi * w[mw][m];
+                    }
                 }
             }
             if (cor) {
@@ -242,6 +248,7 @@ struct WavePatch {
                 for (int mw = 0; mw < MWAVES; mw++) {
                     const TW sa = fabs(s[mw]);
                     coef[mw] = mul_rn(RP::FWAVE ? sgn1(s[mw]) : sa, sub_rn(TW(1), mul_rn(sa, dave)));
+                    if constexpr (F32) coef[mw] = mul_rn(coef[mw], wlim[mw]);
                 }
 #pragma unroll
                 for (int m = 0; m < MEQN; m++) {
@@ -270,17 +277,20 @@ struct WavePatch {
             const auto e = RP::template split_state<IXY>(
                 st, [&](int right) { return (TW)Q()[right ? cR : cL]; }, aux, P);
             TW bm[MEQN], bp[MEQN];
-            RP::template split<IXY>(e, 1, aux, am, bm, bp);
 #pragma unroll
-            for (int m = 0; m < MEQN; m++) {
-                T()[(0 * MEQN + m) * NI + k] = TW(0.5) * dlo * bm[m];
-                T()[(1 * MEQN + m) * NI + k] = TW(0.5) * dlo * bp[m];
-            }
-            RP::template split<IXY>(e, 2, aux, ap, bm, bp);
+            for (int part = 0; part < 2; part++) {                // amdq, then apdq
+                TW* as = part ? ap : am;
+                const TW half = TW(0.5) * (part ? dhi : dlo);
+                if constexpr (F32) {                              // the split is linear: scale what goes in
 #pragma unroll
-            for (int m = 0; m < MEQN; m++) {
-                T()[(2 * MEQN + m) * NI + k] = TW(0.5) * dhi * bm[m];
-                T()[(3 * MEQN + m) * NI + k] = TW(0.5) * dhi * bp[m];
+                    for (int m = 0; m < MEQN; m++) as[m] = half * as[m];
+                }
+                RP::template split<IXY>(e, 1 + part, aux, as, bm, bp);
+#pragma unroll
+                for (int m = 0; m < MEQN; m++) {
+                    T()[((2 * part + 0) * MEQN + m) * NI + k] = F32 ? bm[m] : half * bm[m];
+                    T()[((2 * part + 1) * MEQN + m) * NI + k] = F32 ? bp[m] : half * bp[m];
+                }
             }
         }
     }

@@ -149,7 +149,13 @@ __device__ __forceinline__ T limiter_phi(int mthlim, T r)
     case 1: return dmax1(T(0), dmin1(T(1), r));
     case 2: return dmax1(dmax1(T(0), dmin1(T(1), T(2) * r)), dmin1(T(2), r));
     case 3: return (r + fabs(r)) / (T(1) + fabs(r));
-    case 4: { T c = (T(1) + r) / T(2); return dmax1(T(0), dmin1(dmin1(c, T(2)), T(2) * r)); }
+    case 4:
+        if constexpr (sizeof(T) == 4) {
+            return fmaxf(0.0f, fminf(fminf(fmaf(0.5f, r, 0.5f), 2.0f), 2.0f * r));   // one instruction each
+        } else {
+            T c = (T(1) + r) / T(2);
+            return dmax1(T(0), dmin1(dmin1(c, T(2)), T(2) * r));
+        }
     case 5: return r;
     case 6: { T th = T((double)1.3f); return dmax1(T(0), dmin1(dmin1(th * r, (T(1) + r) / T(2)), th)); }
     default: return T(1);

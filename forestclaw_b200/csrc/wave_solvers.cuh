@@ -40,9 +40,9 @@ template <int IXY> struct Dir { static constexpr int mu = IXY == 1 ? 1 : 2, mv =
 // applications/clawpack/shallow/2d/rp/clawpack46_rpn2.f:1-247, clawpack46_rpt2.f:248-321
 // ---------------------------------------------------------------------------
 struct WaveShallowRoe {
-    static constexpr int MEQN = 3, MWAVES = 3, MAUX = 0, NPRE = 6, NW = 7, NFL = 3, NCONST = 0;
+    static constexpr int MEQN = 3, MWAVES = 3, MAUX = 0, NPRE = 3, NW = 7, NFL = 3, NCONST = 0;
     static constexpr bool FWAVE = false, DEPTH = true, EXACT = false;
-    enum { P_RS = 0, P_N1 = 1, P_N2 = 2, P_U1 = 3, P_U2 = 4, P_C = 5 };   // sqrt h, (hu, hv)/sqrt h, (hu, hv)/h, sqrt gh
+    enum { P_RS = 0, P_N1 = 1, P_N2 = 2 };   // sqrt h, (hu, hv)/sqrt h
     template <int IXY> __host__ __device__ static constexpr int wp(int mw, int m)
     {
         return mw == 0 ? m : mw == 2 ? 4 + m : m == Dir<IXY>::mv ? 3 : -1;
@@ -51,8 +51,12 @@ struct WaveShallowRoe {
     {
         const T rs = sqrt(q[0]);
         c[P_RS] = rs; c[P_N1] = q[1] / rs; c[P_N2] = q[2] / rs;
-        c[P_U1] = q[1] / q[0]; c[P_U2] = q[2] / q[0];
-        c[P_C] = sqrt(P.grav * q[0]);
+    }
+    // Whether |hu|/h can reach sqrt(g h): false only where hu^2 is clearly below g h^3 (one per
+    // cent, far beyond rounding), so the caller's exact test of hu/h -+ sqrt(g h) would fail too.
+    template <typename T> __device__ __forceinline__ static bool fast(T h, T hu, T grav)
+    {
+        return !(hu * hu < T(0.99) * (grav * (h * (h * h))));
     }
     // FP64 cell fluxes of the FP32-wave form: f_x = (hu, F0, F2), f_y = (hv, F2, F1)
     __device__ static void flux_planes(const double* q, const WavePar<float>&, double grav, double* f)
@@ -74,7 +78,7 @@ struct WaveShallowRoe {
     {
         (void)aL; (void)aR;
         constexpr int mu = Dir<IXY>::mu, mv = Dir<IXY>::mv;
-        constexpr int NN = IXY == 1 ? P_N1 : P_N2, NT = IXY == 1 ? P_N2 : P_N1, UN = IXY == 1 ? P_U1 : P_U2;
+        constexpr int NN = IXY == 1 ? P_N1 : P_N2, NT = IXY == 1 ? P_N2 : P_N1;
         // :91-99
         const T h = (qL[0] + qR[0]) / T(2);
         const T hsq2 = cL(P_RS) + cR(P_RS);
@@ -85,30 +89,34 @@ struct WaveShallowRoe {
         const T d1 = qR[0] - qL[0], d2 = qR[mu] - qL[mu], d3 = qR[mv] - qL[mv];
         const T a1 = ((u + a) * d1 - d2) / (T(2) * a);
         const T a2 = -(v * d1) + d3;
-        const T a3 = (-((u - a) * d1) + d2) / (T(2) * a);
+        T a3;
+        if constexpr (sizeof(T) == 4) { a3 = d1 - a1; }           // the two acoustic strengths sum to d1
+        else { a3 = (-((u - a) * d1) + d2) / (T(2) * a); }
         st.a1 = a1; st.a2 = a2; st.a3 = a3; st.u = u; st.v = v; st.a = a;
         const T sl = u - a, sr = u + a;
         const T w0n = a1 * sl, w0t = a1 * v, w2n = a3 * sr, w2t = a3 * v;
-        // entropy fix :170-229
+        // entropy fix :170-229.  The characteristic speeds of the cells and the middle states (a
+        // quotient and a square root each) decide only supersonic and transonic interfaces, and
+        // are formed only where one is possible.
         T am[3] = {T(0), T(0), T(0)};
-        const T s0 = cL(UN) - cL(P_C);
-        if (!(s0 > T(0) && sl > T(0))) {
+        auto speed = [&](T h_, T hu_, T sign) { return hu_ / h_ + sign * sqrt(P.grav * h_); };
+        if (!(sl > T(0) && speed(qL[0], qL[mu], T(-1)) > T(0))) {
             const T h1 = qL[0] + a1, hu1 = qL[mu] + w0n;
-            const T s1 = hu1 / h1 - sqrt(P.grav * h1);
-            T sf;
-            if (s0 < T(0) && s1 > T(0)) sf = s0 * ((s1 - sl) / (s1 - s0));
-            else if (sl < T(0)) sf = sl;
-            else sf = T(0);
+            T sf = sl < T(0) ? sl : T(0);
+            if (hu1 > T(0) && fast(h1, hu1, P.grav)) {
+                const T s1 = speed(h1, hu1, T(-1)), s0 = speed(qL[0], qL[mu], T(-1));
+                if (s0 < T(0) && s1 > T(0)) sf = s0 * ((s1 - sl) / (s1 - s0));
+            }
             am[0] = sf * a1; am[mu] = sf * w0n; am[mv] = sf * w0t;
             if (!(u > T(0))) {
                 am[mv] = am[mv] + u * a2;
-                const T s03 = cR(UN) + cR(P_C);
                 const T h3 = qR[0] - a3, hu3 = qR[mu] - w2n;
-                const T s3 = hu3 / h3 + sqrt(P.grav * h3);
-                bool third = true;
-                if (s3 < T(0) && s03 > T(0)) sf = s3 * ((s03 - sr) / (s03 - s3));
-                else if (sr < T(0)) sf = sr;
-                else third = false;
+                sf = sr;
+                bool third = sr < T(0);
+                if (hu3 < T(0) && fast(h3, hu3, P.grav)) {
+                    const T s3 = speed(h3, hu3, T(1)), s03 = speed(qR[0], qR[mu], T(1));
+                    if (s3 < T(0) && s03 > T(0)) { sf = s3 * ((s03 - sr) / (s03 - s3)); third = true; }
+                }
                 if (third) {
                     am[0] = am[0] + sf * a3; am[mu] = am[mu] + sf * w2n; am[mv] = am[mv] + sf * w2t;
                 }
@@ -152,6 +160,16 @@ struct WaveShallowRoe {
         const T u = e.u, v = e.v, a = e.a;
         const T a1 = ((v + a) * asdq[0] - asdq[mv]) / (T(2) * a);
         const T a2 = asdq[mu] - u * asdq[0];
+        if constexpr (sizeof(T) == 4) {
+            // FP32: a1 + a3 = asdq_0, and the common factors of the components taken out
+            const T a3 = asdq[0] - a1, s0 = v - a, s2 = v + a;
+            const T m0 = fmin(s0, T(0)) * a1, m1 = fmin(v, T(0)) * a2, m2 = fmin(s2, T(0)) * a3;
+            const T p0 = fmax(s0, T(0)) * a1, p1 = fmax(v, T(0)) * a2, p2 = fmax(s2, T(0)) * a3;
+            bm[0] = m0 + m2; bp[0] = p0 + p2;
+            bm[mu] = u * bm[0] + m1; bp[mu] = u * bp[0] + p1;
+            bm[mv] = m0 * s0 + m2 * s2; bp[mv] = p0 * s0 + p2 * s2;
+            return;
+        }
         const T a3 = (-((v - a) * asdq[0]) + asdq[mv]) / (T(2) * a);
         const T sb0 = v - a, sb1 = v, sb2 = v + a;
         const T m0 = dmin1(sb0, T(0)), m1 = dmin1(sb1, T(0)), m2 = dmin1(sb2, T(0));
@@ -228,24 +246,31 @@ struct WaveShallowFWave {
         const T s1 = fmin(uL - gL, uhat - chat);
         const T s3 = fmax(uR + gR, uhat + chat);
         st.b1 = -(fd2 - s3 * fd1) / (s3 - s1);
-        st.b3 = (fd2 - s1 * fd1) / (s3 - s1);
+        if constexpr (sizeof(T) == 4) { st.b3 = fd1 - st.b1; }    // the two strengths sum to fd1
+        else { st.b3 = (fd2 - s1 * fd1) / (s3 - s1); }
         st.b2 = fd3 - st.b1 * vL - st.b3 * vR;
         st.s1 = s1; st.s3 = s3; st.vL = vL; st.vR = vR;
-        // speeds of the transverse solve (rpt2_tsunami.f90:60-118), the same for both fluctuations
+        // speeds of the transverse solve (rpt2_tsunami.f90:60-118), the same for both
+        // fluctuations; between wet cells its celerity is chat, and in FP32 its velocities are
+        // averaged with the weights at hand (sqrt(g h) in place of sqrt h)
         const bool dl = hL < P.drytol, dr = hR < P.drytol;
         const T hl = dl ? T(0) : hL, hr = dr ? T(0) : hR;
         st.dry = hl <= P.drytol && hr <= P.drytol;
-        const T ul = dl ? T(0) : uL, vl = dl ? T(0) : vL, ur = dr ? T(0) : uR, vr = dr ? T(0) : vR;
-        const T rl = dl ? T(0) : cL(P_RS), rr = dr ? T(0) : cR(P_RS);
-        const T rs = rr + rl;
-        const T vhat = (vr * rr) / rs + (vl * rl) / rs;
-        const T uhatt = (ur * rr) / rs + (ul * rl) / rs;
-        const T hhat = (hr + hl) / T(2);
-        const T ct = sqrt(grav * hhat);
-        const T s1l = vl - (dl ? T(0) : gL), s3r = vr + (dr ? T(0) : gR);
-        st.t1 = fmin(vhat - ct, s1l);
-        st.t3 = fmax(vhat + ct, s3r);
-        st.t2 = uhatt;
+        const bool wet = !dl && !dr;
+        T vhat, ct = chat;
+        if (sizeof(T) == 4 && wet) {
+            vhat = (gL * vL + gR * vR) / (gR + gL);
+            st.t2 = uhat;
+        } else {
+            const T ul = dl ? T(0) : uL, vl = dl ? T(0) : vL, ur = dr ? T(0) : uR, vr = dr ? T(0) : vR;
+            const T rl = dl ? T(0) : cL(P_RS), rr = dr ? T(0) : cR(P_RS);
+            const T rs = rr + rl;
+            vhat = (vr * rr) / rs + (vl * rl) / rs;
+            st.t2 = (ur * rr) / rs + (ul * rl) / rs;
+            if (!wet) ct = sqrt(grav * ((hr + hl) / T(2)));
+        }
+        st.t1 = fmin(vhat - ct, (dl ? T(0) : vL) - (dl ? T(0) : gL));
+        st.t3 = fmax(vhat + ct, (dr ? T(0) : vR) + (dr ? T(0) : gR));
         expand<IXY>(st, 0, w, s);
         return 0;
     }
@@ -292,9 +317,15 @@ struct WaveShallowFWave {
         }
         const T s1 = e.t1, s2 = e.t2, s3 = e.t3;
         const T d1 = asdq[0], d2 = asdq[mu], d3 = asdq[mv];
-        const T b0 = (s3 * d1 / (s3 - s1)) - (d3 / (s3 - s1));
+        T b0, b2;
+        if constexpr (sizeof(T) == 4) {
+            b0 = (s3 * d1 - d3) / (s3 - s1);
+            b2 = d1 - b0;
+        } else {
+            b0 = (s3 * d1 / (s3 - s1)) - (d3 / (s3 - s1));
+            b2 = (d3 / (s3 - s1)) - (s1 * d1 / (s3 - s1));
+        }
         const T b1 = -(s2 * d1) + d2;
-        const T b2 = (d3 / (s3 - s1)) - (s1 * d1 / (s3 - s1));
         const T g0 = s1 * b0, g1 = s2 * b1, g2 = s3 * b2;
         const bool n0 = signbit(s1), n1 = signbit(s2), n2 = signbit(s3);
         const T m0 = n0 ? g0 : T(0), m1 = n1 ? g1 : T(0), m2 = n2 ? g2 : T(0);
