@@ -30,6 +30,15 @@ __device__ __forceinline__ int group_slot(const LevelGroup& lg, int b)
     return lg.nlev - 1 - k;
 }
 
+// r = (zero ? 0 : r) + v for a register no other thread touches during the launch, without
+// waiting for it: a reduction in L2 (one correctly rounded addition, as here) instead of a load,
+// an addition and a store, whose load each CTA waited for between its barriers.
+__device__ __forceinline__ void accumulate(double* r, bool zero, double v)
+{
+    if (zero) *r = 0.0 + v;
+    else atomicAdd(r, v);
+}
+
 // Host flag of the calling thread: launches through launch_k carry the
 // programmatic-serialization attribute while it is set (ProgrammaticScope).
 bool programmatic_launch();

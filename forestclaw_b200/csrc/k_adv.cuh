@@ -284,8 +284,7 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
         const double dtdyv = dt * dy, dtdxv = dt * dx;
         // registers of a face reset since the last update start from zero
         auto add = [&](int face, int r, double v) {
-            const bool zero = (sp->reg_reset >> ((pd->face_type >> (2 * face)) & 3)) & 1;
-            rg[r] = (zero ? 0.0 : rg[r]) + v;
+            accumulate(&rg[r], (sp->reg_reset >> ((pd->face_type >> (2 * face)) & 3)) & 1, v);
         };
         for (int it = tid; it < MY + MX; it += NT) {
             double fm, fp;

@@ -473,10 +473,7 @@ wave_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __
             const double el = (face < 2) ? dy : dx;
             const int base = (face == 0) ? G::R_EF0 : (face == 1) ? G::R_EF1 : (face == 2) ? G::R_EF2 : G::R_EF3;
             const bool zero = (sp->reg_reset >> ((pd->face_type >> (2 * face)) & 3)) & 1;
-            for (int m = 0; m < MEQN; m++) {
-                double* r = &rg[base + j + m * n + k * n * MEQN];
-                *r = (zero ? 0.0 : *r) + dt * el * fl[m];
-            }
+            for (int m = 0; m < MEQN; m++) accumulate(&rg[base + j + m * n + k * n * MEQN], zero, dt * el * fl[m]);
         }
     }
     if (bad && sp->status) atomicOr(sp->status, bad);
@@ -580,8 +577,7 @@ wave_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __
         const int reset = sp->reg_reset, ft = pd->face_type;
         // registers of a face reset since the last update start from zero
         auto add = [&](int face, int r, double v) {
-            const bool zero = (reset >> ((ft >> (2 * face)) & 3)) & 1;
-            rg[r] = (zero ? 0.0 : rg[r]) + v;
+            accumulate(&rg[r], (reset >> ((ft >> (2 * face)) & 3)) & 1, v);
         };
         for (int it = tid; it < (MY + MX) * MEQN; it += NT) {
             if (it < MY * MEQN) {
