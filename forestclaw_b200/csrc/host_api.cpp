@@ -1047,7 +1047,7 @@ extern "C" int fc2d_b200_create(const fc2d_b200_options_t* opt, fc2d_b200_solver
     {
         using S = fc2d_b200_solver;
         static_assert(S::BLK_PARAMS % alignof(StepParams) == 0, "parameter blocks follow aligned");
-        const size_t bytes = S::BLK_PARAMS + sizeof(StepParams) * S::PCAP;
+        const size_t bytes = S::BLK_PARAMS + sizeof(StepParams) * S::PCAP + 16;
         CK(cudaMalloc(&s->block_dev, bytes));
         CK(cudaMemset(s->block_dev, 0, S::BLK_PARAMS));
         CK(cudaMallocHost(&s->block_host, bytes));
@@ -1362,10 +1362,13 @@ static int begin_cfl(fc2d_b200_solver* s)
     return 0;
 }
 // The status word and CFL maxima of the work on the stream, to result_host.
+static size_t result_bytes(const fc2d_b200_solver* s)
+{
+    return (fc2d_b200_solver::BLK_CFL + 8 * (size_t)s->ncfl + 15) / 16 * 16;
+}
 static cudaError_t fetch_result(fc2d_b200_solver* s)
 {
-    return cudaMemcpyAsync(s->result_host, s->block_dev, fc2d_b200_solver::BLK_CFL + 8 * (size_t)s->ncfl,
-                           cudaMemcpyDeviceToHost, s->st);
+    return cudaMemcpyAsync(s->result_host, s->block_dev, result_bytes(s), cudaMemcpyDeviceToHost, s->st);
 }
 
 // The kernels' failure reports (device status word) as an error message, or "".
@@ -1614,13 +1617,13 @@ static int advance_launch(fc2d_b200_solver_t* s, double t, double dt)
     CK(cudaEventRecord(ev[0], s->st));
     const int nupd = s->n_upd;
     // the step block up, the launches, the result down
-    auto issue = [&](bool captured) -> int {
-        CK(cudaMemcpyAsync(s->block_dev, s->block_host, fc2d_b200_solver::BLK_PARAMS + sizeof(StepParams) * nupd,
-                           cudaMemcpyHostToDevice, s->st));
-        ProgrammaticScope pscope(s->programmatic, captured);
+    auto issue = [&]() -> int {
+        ProgrammaticScope pscope(s->programmatic);
+        launch_step_begin(s->block_dev, s->block_host,
+                          (fc2d_b200_solver::BLK_PARAMS + sizeof(StepParams) * nupd + 15) / 16 * 16, s->st);
         int r = traverse_advance(s, t, dt);
         if (r) return r;
-        CK(fetch_result(s));
+        launch_step_end(s->result_host, s->block_dev, result_bytes(s), s->st);
         return 0;
     };
     // pass 2: the launches, captured once per forest into a CUDA graph and replayed
@@ -1629,7 +1632,7 @@ static int advance_launch(fc2d_b200_solver_t* s, double t, double dt)
         if (s->graph_stale || !s->graph_exec || s->graph_nupd != nupd) {
             cudaGraph_t g = nullptr;
             CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
-            rc = issue(true);
+            rc = issue();
             cudaError_t ec = cudaStreamEndCapture(s->st, &g);
             if (rc) { if (g) cudaGraphDestroy(g); s->fill = true; return rc; }
             if (ec != cudaSuccess) { s->fill = true; return fail(FC2D_B200_ECUDA, std::string("graph capture: ") + cudaGetErrorString(ec)); }
@@ -1657,7 +1660,7 @@ static int advance_launch(fc2d_b200_solver_t* s, double t, double dt)
         }
         CK(cudaGraphLaunch(s->graph_exec, s->st));
     } else {
-        rc = issue(false);
+        rc = issue();
     }
     s->fill = true;
     if (rc) return rc;

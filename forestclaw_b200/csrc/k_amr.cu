@@ -19,17 +19,9 @@
 
 namespace fcb {
 
-static thread_local bool tl_programmatic = false, tl_after_copy = false;
-void set_programmatic_launch(bool on, bool after_copy)
-{
-    tl_programmatic = on;
-    tl_after_copy = after_copy;
-}
-bool programmatic_launch()
-{
-    if (tl_after_copy) { tl_after_copy = false; return false; }
-    return tl_programmatic;
-}
+static thread_local bool tl_programmatic = false;
+void set_programmatic_launch(bool on) { tl_programmatic = on; }
+bool programmatic_launch() { return tl_programmatic; }
 
 static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
@@ -480,6 +472,16 @@ __global__ void k_reset_sync(double* __restrict__ regs, const PatchDesc* __restr
     if (t < reset_sync_items(np, mx, my, meqn)) reset_sync_at(regs, desc, p0, mx, my, meqn, nreg, minlevel, maxl, t);
 }
 
+// The step block up and the result down, by a thread per 16 bytes over the host link: as copy
+// nodes they cost the step's graph a hand-over between copy engine and compute on either side
+// (about 3 us each); as kernels they are links of the programmatic chain.
+__global__ void __launch_bounds__(512) k_step_copy(uint4* __restrict__ to, const uint4* __restrict__ from, int n)
+{
+    grid_dependency_wait();       // programmatic launch: the previous grid's writes are visible
+    grid_launch_dependents();
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) to[k] = from[k];
+}
+
 // Per-patch, per-field Kahan sums of q*dx*dy over interior cells in (j, i) order.
 __global__ void k_patch_mass(const double* __restrict__ q, const PatchDesc* __restrict__ desc, int mx, int my,
                              int mbc, int meqn, double* __restrict__ out, const double* __restrict__ areas)
@@ -786,6 +788,15 @@ void launch_reset_sync(const Dims& d, double* regs, const PatchDesc* desc, int p
     if (np > 0)
         launch_k(k_reset_sync, nblk(n, 256), 256, 0, st, regs, desc, p0, np, d.mx, d.my, d.meqn, d.nreg(), minlevel,
                  maxl);
+}
+void launch_step_begin(void* block_dev, const void* block_host, size_t bytes, cudaStream_t st)
+{
+    const int n = (int)(bytes / 16), blocks = n <= 512 ? 1 : n <= 8 * 512 ? nblk(n, 512) : 8;
+    launch_k(k_step_copy, blocks, 512, 0, st, (uint4*)block_dev, (const uint4*)block_host, n);
+}
+void launch_step_end(void* result_host, const void* block_dev, size_t bytes, cudaStream_t st)
+{
+    launch_k(k_step_copy, 1, 128, 0, st, (uint4*)result_host, (const uint4*)block_dev, (int)(bytes / 16));
 }
 void launch_patch_mass(const Dims& d, const double* q, const PatchDesc* desc, int np, double* out, cudaStream_t st,
                        const double* area)

@@ -8,13 +8,13 @@
 namespace fcb {
 
 // Programmatic dependent launch of the advance's kernels (fcb_launch.cuh): on for the
-// calling thread while a ProgrammaticScope lives.  after_copy: the scope's first kernel
-// follows a copy, not a kernel, and is launched plainly.
-void set_programmatic_launch(bool on, bool after_copy);
-bool programmatic_launch();          // for the next launch
+// calling thread while a ProgrammaticScope lives.
+void set_programmatic_launch(bool on);
+bool programmatic_launch();
 struct ProgrammaticScope {
-    ProgrammaticScope(bool on, bool after_copy) { set_programmatic_launch(on, after_copy); }
-    ~ProgrammaticScope() { set_programmatic_launch(false, false); }
+    bool prev;
+    explicit ProgrammaticScope(bool on) : prev(programmatic_launch()) { set_programmatic_launch(on); }
+    ~ProgrammaticScope() { set_programmatic_launch(prev); }
 };
 
 struct Dims {
@@ -112,6 +112,11 @@ void launch_sync(const Dims& d, double* q, const double* regs, const PatchDesc* 
 // over the patches of levels [minlevel, maxl].
 void launch_reset_sync(const Dims& d, double* regs, const PatchDesc* desc, int p0, int np, int minlevel, int maxl,
                        cudaStream_t st);
+
+// The step block of an advance from page-locked host memory to the device, and its result back
+// (bytes: multiples of 16), by kernels of the step's own chain.
+void launch_step_begin(void* block_dev, const void* block_host, size_t bytes, cudaStream_t st);
+void launch_step_end(void* result_host, const void* block_dev, size_t bytes, cudaStream_t st);
 
 // ---- diagnostics / regrid (k_amr.cu) -------------------------------------------
 // area (manifold, else null): the cell areas weight q instead of dx dy
