@@ -2785,8 +2785,12 @@ extern "C" int fc2d_b200_set_variant(fc2d_b200_solver_t* s, int v)
     return 0;
 }
 
-// Time every variant on the current forest -- one launch per level, as a
-// subcycled step issues them -- and keep the fastest.  The timed launches run
+// Time every variant on the update launches of a coarse step of the current forest and keep
+// the fastest.  A subcycled step updates levels [l, finest] together, in one launch: the group
+// down to level l, 2^(l - coarsest - 1) times (the coarsest once; counted 16 times at most).
+// (Timed level by level, variants that are quick on a few patches won forests whose merged
+// launches they slow down: radial dam, levels 3-7, 942 us a step against 870.)  Reported per
+// pass over all levels: a step's time by its share of patches.  The timed launches run
 // with dt = 0 and neither store fluxes, accumulate waves, save q nor count
 // Newton iterations, so they do all of the update's arithmetic but leave q,
 // the registers and the statistics as they were.
@@ -2803,13 +2807,21 @@ extern "C" int fc2d_b200_autotune(fc2d_b200_solver_t* s, int reps, int* best_out
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
+    struct Group { int p0, np, count; };
+    std::vector<Group> groups;
+    double updates = 0;                           // patches updated in the timed step
+    for (int l = f.minlevel_present; l <= f.maxlevel_present; l++) {
+        if (!s->o.subcycle && l > f.minlevel_present) break;
+        const int p0 = f.lev_off[l], below = l - f.minlevel_present;
+        groups.push_back({p0, f.lev_off[f.maxlevel_present + 1] - p0, below == 0 ? 1 : 1 << std::min(below - 1, 4)});
+        updates += (double)groups.back().np * groups.back().count;
+    }
     auto pass = [&](const Step2Variant* v) -> cudaError_t {
-        for (int l = 0; l <= 32; l++) {
-            const int p0 = f.lev_off[l], np = f.lev_off[l + 1] - p0;
-            if (np <= 0) continue;
-            cudaError_t e = v->fn(s->q, s->qlast, s->aux, s->regs, s->desc, p0, np, s->tune_params, one, s->cfl_dev, s->st);
-            if (e != cudaSuccess) return e;
-        }
+        for (const Group& g : groups)
+            for (int k = 0; k < g.count; k++) {
+                cudaError_t e = v->fn(s->q, s->qlast, s->aux, s->regs, s->desc, g.p0, g.np, s->tune_params, one, s->cfl_dev, s->st);
+                if (e != cudaSuccess) return e;
+            }
         return cudaSuccess;
     };
     int best = s->var;
@@ -2824,14 +2836,17 @@ extern "C" int fc2d_b200_autotune(fc2d_b200_solver_t* s, int reps, int* best_out
         if (err == cudaSuccess) err = cudaEventSynchronize(e1);
         float ms = 0.0f;
         if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, e0, e1);
-        const double per = (double)ms / reps;
+        const double per = (double)ms / reps * f.np() / updates;
         if (ms_out) ms_out[v] = per;
         if (err == cudaSuccess && per < best_ms) { best_ms = per; best = v; }
     }
     // then per level: a level's patch count decides how its CTAs fill the waves
     // of the device, so a level takes another variant where that is clearly faster
-    // on it alone (by 5 %: the forest changes between regrids, and a small level's
-    // launch is a few microseconds); each level's timing covers at least ~0.3 ms
+    // on it alone: by 5 % (the forest changes between regrids) and by a launch, since
+    // consecutive levels share a launch only with one variant (on the radial dam,
+    // levels 3-7, a choice by 5 % alone split off small levels and took 978 us a step
+    // against 917 with one variant); each level's timing covers at least ~0.3 ms
+    constexpr double LAUNCH_MS = 0.004;
     auto time_level = [&](const Step2Variant* x, int p0, int np, int n, double& per) -> cudaError_t {
         cudaError_t e = x->fn(s->q, s->qlast, s->aux, s->regs, s->desc, p0, np, s->tune_params, one, s->cfl_dev, s->st);
         if (e == cudaSuccess) e = cudaEventRecord(e0, s->st);
@@ -2854,7 +2869,7 @@ extern "C" int fc2d_b200_autotune(fc2d_b200_solver_t* s, int reps, int* best_out
         const int n = std::max(reps, std::min(64, (int)(0.3 / std::max(est, 1e-3))));
         if (err == cudaSuccess) err = time_level(s->vars[best], p0, np, n, ref);
         lev_best[l] = best;
-        double lbest = 0.95 * ref;
+        double lbest = 0.95 * ref - LAUNCH_MS;
         for (int v = 0; v < (int)s->vars.size() && err == cudaSuccess; v++) {
             if (v == best) continue;
             double per = 0.0;

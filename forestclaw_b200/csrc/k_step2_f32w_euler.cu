@@ -8,11 +8,11 @@ namespace fcb {
 const Step2Variant* step2_table_f32w_euler(int* n)
 {
     static const Step2Variant table[] = {
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 352, 2, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 384, 2, float, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 352, 2, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 352, 1, float, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 384, 2, float, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 352, 2, float, 0),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 352, 1, float, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 8, 128, 6, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 8, 128, 5, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 8, 128, 4, float, 4),

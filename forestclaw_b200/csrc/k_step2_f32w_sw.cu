@@ -9,21 +9,21 @@ namespace fcb {
 const Step2Variant* step2_table_f32w_sw(int* n)
 {
     static const Step2Variant table[] = {
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 384, 3, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 3, float, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 2, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 384, 2, float, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 3, float, 0),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 2, float, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 384, 3, float, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 384, 2, float, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 8, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 6, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 4, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 8, float, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 6, float, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 384, 3, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 3, float, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 2, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 384, 2, float, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 3, float, 0),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 2, float, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 384, 3, float, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 384, 2, float, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 8, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 6, float, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 4, float, 4),

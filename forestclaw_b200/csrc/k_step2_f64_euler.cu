@@ -8,9 +8,9 @@ namespace fcb {
 const Step2Variant* step2_table_f64_euler(int* n)
 {
     static const Step2Variant table[] = {
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 352, 1, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 384, 1, double, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 352, 1, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 352, 1, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 16, 384, 1, double, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 8, 128, 4, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 8, 128, 3, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_EULER_EXACT, WaveEulerExact, 8, 128, 2, double, 4),

@@ -9,26 +9,26 @@ namespace fcb {
 const Step2Variant* step2_table_f64_sw(int* n)
 {
     static const Step2Variant table[] = {
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 2, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 384, 2, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 2, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 1, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 384, 2, double, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 2, double, 0),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 16, 352, 1, double, 0),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 4, double, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 5, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 6, double, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 4, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 5, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 4, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 6, double, 0),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 2, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_ROE, WaveShallowRoe, 8, 128, 4, double, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 384, 2, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 2, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 1, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 384, 2, double, 0),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 2, double, 0),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 16, 352, 1, double, 0),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 4, double, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 5, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 6, double, 4),
-        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 4, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 5, double, 4),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 4, double, 4),
         FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 6, double, 0),
+        FCB_WAVE_VARIANT(FC2D_B200_PREC_FP64, FC2D_B200_RP_SW_FWAVE, WaveShallowFWave, 8, 128, 4, double, 0),
     };
     *n = (int)(sizeof(table) / sizeof(table[0]));
     return table;
