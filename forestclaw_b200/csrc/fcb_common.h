@@ -68,6 +68,11 @@ struct StepParams {
     // face type t: 0 boundary, 1 half, 2 same, 3 double): the update's first
     // accumulation into such a face's registers starts from zero instead of reading them.
     int reg_reset;
+    // Time interpolation of this level inside an advance (fclaw2d_timeinterp), or null: patches
+    // with finer neighbours also write qlast + ti_alpha (q - qlast) of their band of width mbc.
+    // As a kernel of its own it read both arrays back, a launch per coarse update.
+    double* qinterp;
+    double ti_alpha;
 };
 
 // Kernel-side failures reported through the status word (read by the host after a step).

@@ -303,6 +303,8 @@ struct fc2d_b200_solver {
     StepParams* params_dev = nullptr;
     StepParams* params_host = nullptr;
     int n_upd = 0;
+    int level_slot[33] = {};                       // parameter block of each level's latest update
+    bool in_advance = false;                       // traversing an advance
     bool emit = true;                              // false: host traversal only (fill parameters)
     bool fill = true;                              // fill params_host / count statistics
     // CUDA graph of one fclaw2d_advance_all_levels for the current forest
@@ -557,6 +559,8 @@ static StepParams make_params(const fc2d_b200_solver* s, int level, double t, do
     sp.inst_dt = s->insts.empty() ? nullptr : s->inst_dt_dev;
     sp.status = s->status_dev;
     sp.reg_reset = 0;
+    sp.qinterp = nullptr;                          // set where the advance asks for the time interpolation
+    sp.ti_alpha = 0.0;
     if (s->o.app == FC2D_B200_APP_SWIRL && s->o.tperiod != 0.0) {
         const double pi = 4.0 * std::atan(1.0), pi2 = 2.0 * pi;
         sp.vt = std::cos(pi2 * (t + dt / 2.0) / s->o.tperiod);
@@ -627,6 +631,7 @@ static int update_level(fc2d_b200_solver* s, int level, double t, double dt)
     if (s->n_upd >= fc2d_b200_solver::PCAP) return fail(FC2D_B200_EINVAL, "too many level updates in one advance");
     flush_timeinterp(s);                              // it reads q of levels this update may write
     const int slot = s->n_upd++;
+    s->level_slot[level] = slot;
     if (s->fill) {
         StepParams& sp = s->params_host[slot];
         sp = make_params(s, level, t, dt);
@@ -895,6 +900,16 @@ static void time_sync(fc2d_b200_solver* s, int minlevel, int maxlevel, bool defe
 static void timeinterp(fc2d_b200_solver* s, int level, double alpha)
 {
     if (level < 0 || level > 31 || !s->lr[level].ti_n) return;
+    if (s->in_advance && !s->part) {
+        // the level's update, issued just before, writes the band itself (on a partitioned
+        // forest the band of other ranks' patches is formed here, after the halo exchange)
+        if (s->fill) {
+            StepParams& sp = s->params_host[s->level_slot[level]];
+            sp.qinterp = s->qinterp;
+            sp.ti_alpha = alpha;
+        }
+        return;
+    }
     (void)flush_updates(s);
     fc2d_b200_solver::PendingTimeInterp& g = s->pend_ti;
     if (g.active && level == g.lev_hi + 1) {        // the lists of consecutive levels are contiguous
@@ -1573,6 +1588,11 @@ static int traverse_advance(fc2d_b200_solver* s, double t, double dt)
     s->n_upd = 0;
     s->pend.active = false;
     s->pend_ti.active = false;
+    struct Advancing {
+        bool& on;
+        explicit Advancing(bool& b) : on(b) { on = true; }
+        ~Advancing() { on = false; }
+    } advancing(s->in_advance);
     const int nfine = ts[maxlevel].total_steps;
     for (int nf = 0; nf < nfine; nf++) {
         int rc = advance_level(s, ts, maxlevel, nf);

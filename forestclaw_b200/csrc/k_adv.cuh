@@ -310,6 +310,7 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
     // ---- q over i,j = 1-mbc..mx+mbc-1 (clawpack46_step2_wrap.f:107-125); faces of column or
     // row 0 are no sweep's and have no flux ----
     double* qg = q + (size_t)p * NXY;
+    double* qi = sp->qinterp && (pd->flags & PATCH_HAS_FINE_NBR) ? sp->qinterp + (size_t)p * NXY : nullptr;
     for (int c = tid; c < NXY; c += NT) {
         const int jc = c / NX, ic = c - jc * NX;
         if (ic <= NX - 2 && jc <= NY - 2) {
@@ -322,10 +323,12 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
                 X.template flux<2>(c + NX, jc + 1, ic, gt, none);
                 if (jc >= 1) X.template flux<2>(c, jc, ic, none, gb);
             }
-            double v = Q[c];
+            const double old = Q[c];
+            double v = old;
             if (X.M.mcapa() == 0) v = v - X.dtdx * (fr - fl) - X.dtdy * (gt - gb);
             else v = v - (X.dtdx * (fr - fl) + X.dtdy * (gt - gb)) / X.A(X.M.mcapa() - 1)[c];
             qg[c] = v;
+            if (qi && in_band(ic, jc, MX, MY, MBC)) qi[c] = add_rn(old, mul_rn(sp->ti_alpha, sub_rn(v, old)));
         } else if (bcc) {
             // cells the update skips keep the step's (corner-fixed) values, as the
             // reference fixes the corners of q in place

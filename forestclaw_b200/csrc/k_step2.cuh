@@ -452,6 +452,13 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     }
 
     // ---- q update over i,j = 1-mbc..mx+mbc-1 (clawpack46_step2_wrap.f:107-125) ----
+    double* qi = sp.qinterp && (pd.flags & PATCH_HAS_FINE_NBR) ? sp.qinterp + (size_t)p * MEQN * NXY : nullptr;
+    auto interpolate = [&](int m, int c, int ic, int jc, double v) {
+        if (qi && in_band(ic, jc, MX, MY, MBC)) {
+            const double old = Qs[m * NXY + c];
+            qi[m * NXY + c] = add_rn(old, mul_rn(sp.ti_alpha, sub_rn(v, old)));
+        }
+    };
     if constexpr (RPHooks<RP>::SRC) {
         // with a user src2 (clawpack46_update, fc2d_clawpack46.cpp:436-441: src2 after
         // step2), every padded cell gets its updated q (cells the update skips keep
@@ -474,7 +481,10 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
             for (int a = 0; a < G::AUXS; a++) ac[a] = As[a * NXY + c];
             RP::src2(MBC, MX, MY, MEQN, qc, pd.xlower, pd.ylower, dx, dy, sp.t, dt, G::AUXS, ac, ic - MBC + 1,
                      jc - MBC + 1);
-            for (int m = 0; m < MEQN; m++) qg[m * NXY + c] = qc[m];
+            for (int m = 0; m < MEQN; m++) {
+                qg[m * NXY + c] = qc[m];
+                interpolate(m, c, ic, jc, qc[m]);
+            }
         }
     } else
     for (int k = tid; k < MEQN * NXY; k += NT) {
@@ -489,6 +499,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
                 v = v - (dtdx * (FMs[b + c + 1] - FPs[b + c]) + dtdy * (GMs[b + c + NX] - GPs[b + c])) /
                             As[(mcapa - 1) * NXY + c];
             qg[k] = v;
+            interpolate(m, c, ic, jc, v);
         }
     }
 

@@ -598,25 +598,25 @@ wave_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __
     // ---- q over i,j = 1-mbc..mx+mbc-1 (clawpack46_step2_wrap.f:107-125); faces of column or
     // row 0 are no sweep's and have no flux ----
     double* qg = q + (size_t)p * MEQN * NXY;
+    double* qi = sp->qinterp && (pd->flags & PATCH_HAS_FINE_NBR) ? sp->qinterp + (size_t)p * MEQN * NXY : nullptr;
     for (int c = tid; c < NXY; c += NT) {
         const int jc = c / NX, ic = c - jc * NX;
         if (ic > NX - 2 || jc > NY - 2) continue;
+        const bool band = qi && in_band(ic, jc, MX, MY, MBC);
 #pragma unroll
         for (int m = 0; m < MEQN; m++) {
             const double fr = jc >= 1 ? X.fm_x(m, ic + 1, jc) : 0.0;
             const double fl = jc >= 1 && ic >= 1 ? X.fp_x(m, ic, jc) : 0.0;
             const double gt = ic >= 1 ? X.gm_y(m, ic, jc + 1) : 0.0;
             const double gb = jc >= 1 && ic >= 1 ? X.gp_y(m, ic, jc) : 0.0;
-            double v = Q[m * NXY + c];
-            if constexpr (G::MAUX > 0 && LIM == 0) {
-                if (X.M.mcapa > 0) {
-                    v = v - (X.dtdx * (fr - fl) + X.dtdy * (gt - gb)) / X.A()[(X.M.mcapa - 1) * NXY + c];
-                    qg[m * NXY + c] = v;
-                    continue;
-                }
-            }
-            v = v - X.dtdx * (fr - fl) - X.dtdy * (gt - gb);
+            const double old = Q[m * NXY + c];
+            double v = old;
+            bool capacity = false;
+            if constexpr (G::MAUX > 0 && LIM == 0) capacity = X.M.mcapa > 0;
+            if (capacity) v = v - (X.dtdx * (fr - fl) + X.dtdy * (gt - gb)) / X.A()[(X.M.mcapa - 1) * NXY + c];
+            else v = v - X.dtdx * (fr - fl) - X.dtdy * (gt - gb);
             qg[m * NXY + c] = v;
+            if (band) qi[m * NXY + c] = add_rn(old, mul_rn(sp->ti_alpha, sub_rn(v, old)));
         }
     }
 

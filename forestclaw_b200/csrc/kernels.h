@@ -93,7 +93,8 @@ void launch_interp(const Dims& d, const GatherSeg<InterpEnt>& s0, const GatherSe
 void launch_phys(const Dims& d, const GatherSeg<PhysEnt>& s0, const GatherSeg<PhysEnt>& s1, const double* bcstate,
                  cudaStream_t st);
 // time interpolation factor of each level (levels 0..31) for a launch over the
-// time-interpolation lists of several levels
+// time-interpolation lists of several levels (inside an advance of one rank the updates
+// write the time-interpolated band themselves, StepParams::qinterp)
 struct LevelAlpha { double a[32]; };
 void launch_timeinterp(const Dims& d, const double* q, const double* qlast, double* qinterp, const int* patches,
                        int npatch, const PatchDesc* desc, const LevelAlpha& alpha, cudaStream_t st);

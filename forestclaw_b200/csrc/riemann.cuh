@@ -12,6 +12,14 @@ template <typename T> __device__ __forceinline__ T dmin1(T a, T b) { return a < 
 template <typename T> __device__ __forceinline__ T dmax1(T a, T b) { return a > b ? a : b; }
 template <typename T> __device__ __forceinline__ T sgn1(T x) { return copysign(T(1), x); }
 
+// Whether padded cell (ic, jc) lies in the band of width mbc inside an mx x my patch that time
+// interpolation fills (fclaw2d_clawpatch46_timeinterp.f:33-70).
+__device__ __forceinline__ bool in_band(int ic, int jc, int mx, int my, int mbc)
+{
+    return ic >= mbc && ic < mx + mbc && jc >= mbc && jc < my + mbc &&
+           (ic < 2 * mbc || ic >= mx || jc < 2 * mbc || jc >= my);
+}
+
 // Correctly rounded, uncontracted multiply / add.  The FP32-wave units are built with
 // FMA contraction; the second-order correction must not be contracted, or the
 // exactly opposite terms of the waves at a reflecting wall leave the rounding
