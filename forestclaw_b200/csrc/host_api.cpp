@@ -223,7 +223,8 @@ struct fc2d_b200_solver {
     DevVec<int> aux_src_dev;                       // regrid: where each new patch's aux comes from
     DevVec<double> aux_staged_dev;                 // regrid: aux of new patches from the app's setaux
     TableArena arena;                              // the tables below, on the device
-    DevView<FillOp> t_copy;                        // copy2ghost region ops
+    DevView<FillOp> t_copy;                        // copy2ghost region ops (cubed sphere)
+    DevView<int> t_nbr;                            // copy2ghost neighbours (bricks)
     DevView<FillOp> t_avg;                         // average2ghost region ops
     double* area = nullptr;                        // cubed sphere: cell areas per patch (Dims::narea per patch)
     bool sphere = false;                           // the cubed-sphere app (manifold, 6 blocks)
@@ -451,6 +452,8 @@ static int upload_desc_and_tables(fc2d_b200_solver* s)
             v.resize(n);
         };
         filter(T.copy, T.copy_off, [&](const FillOp& e) { return fill[e.dst] != 0; });
+        for (size_t k = 0; k < T.copy_nbr.size(); k++)
+            if (!fill[k / 8]) T.copy_nbr[k] = -1;
         filter(T.avg, T.avg_off, [&](const FillOp& e) { return fill[e.dst] != 0; });
         filter(T.phys, T.phys_off, [&](const PhysEnt& e) { return fill[e.dst / nq] != 0; });
         filter(T.interp, T.interp_off, [&](const InterpEnt& e) { return own[e.dst / nq] == me; });
@@ -480,10 +483,11 @@ static int upload_desc_and_tables(fc2d_b200_solver* s)
         TableArena& A = s->arena;
         auto sz = [](const auto& v) { return TableArena::span(v.size() * sizeof(v[0])); };
         CK(A.wait_copied());
-        CK(A.reserve(sz(hd) + sz(T.copy) + sz(T.avg) + sz(T.interp) + sz(T.phys) + sz(T.ti) + sz(T.sync)));
+        CK(A.reserve(sz(hd) + sz(T.copy) + sz(T.copy_nbr) + sz(T.avg) + sz(T.interp) + sz(T.phys) + sz(T.ti) + sz(T.sync)));
         A.used = 0;
         const DevView<PatchDesc> dv = A.put(hd);       // staged here, then copied into the slab's descriptors
         s->t_copy = A.put(T.copy);
+        s->t_nbr = A.put(T.copy_nbr);
         s->t_avg = A.put(T.avg);
         s->t_interp = A.put(T.interp);
         s->t_phys = A.put(T.phys);
@@ -689,7 +693,9 @@ static GatherSeg<E> seg(const E* table, int off, int n, double* dst, const doubl
 // ghost cells and read interior cells only, so their order does not matter
 static void average_copy_range(fc2d_b200_solver* s, int a, int b, int ca, int cb, int c)
 {
-    GatherSeg<FillOp> a0{nullptr, nullptr, nullptr, 0}, a1 = a0, c0 = a0, c1 = a0;
+    GatherSeg<FillOp> a0{nullptr, nullptr, nullptr, 0}, a1 = a0, f0 = a0, f1 = a0;
+    CopySeg c0{nullptr, 0, 0}, c1 = c0;
+    const int* lev_off = s->forest.lev_off;
     if (lrange(a, b)) {
         const int off = s->lr[a].avg_off, n = s->lr[b].avg_off + s->lr[b].avg_n - off;
         if (n > 0) a0 = seg(s->t_avg.p, off, n, s->q, s->q);
@@ -698,14 +704,17 @@ static void average_copy_range(fc2d_b200_solver* s, int a, int b, int ca, int cb
         a1 = seg(s->t_avg.p, s->lr[c].avg_off, s->lr[c].avg_n, s->qinterp, s->q);
     if (lrange(ca, cb)) {
         const int off = s->lr[ca].copy_off, n = s->lr[cb].copy_off + s->lr[cb].copy_n - off;
-        if (n > 0) c0 = seg(s->t_copy.p, off, n, s->q, s->q);
+        if (n > 0) f0 = seg(s->t_copy.p, off, n, s->q, s->q);
+        if (!s->sphere && lev_off[cb + 1] - lev_off[ca] > 1) c0 = CopySeg{s->q, lev_off[ca], lev_off[cb + 1] - lev_off[ca]};
     }
-    if (c >= 0 && c <= 32 && s->lr[c].copy_n > 0)
-        c1 = seg(s->t_copy.p, s->lr[c].copy_off, s->lr[c].copy_n, s->qinterp, s->qinterp);
-    if (a0.n + a1.n + c0.n + c1.n <= 0) return;
+    if (c >= 0 && c <= 32) {
+        if (s->lr[c].copy_n > 0) f1 = seg(s->t_copy.p, s->lr[c].copy_off, s->lr[c].copy_n, s->qinterp, s->qinterp);
+        if (!s->sphere && lev_off[c + 1] - lev_off[c] > 1) c1 = CopySeg{s->qinterp, lev_off[c], lev_off[c + 1] - lev_off[c]};
+    }
+    if (a0.n + a1.n + f0.n + f1.n + c0.np + c1.np <= 0) return;
     (void)flush_pending(s);
     if (s->fill) s->total_launches++;
-    if (s->emit) launch_average_copy(s->d, a0, a1, c0, c1, s->area, s->st);
+    if (s->emit) launch_average_copy(s->d, a0, a1, f0, f1, c0, c1, s->t_nbr.p, s->area, s->st);
 }
 static void phys_range(fc2d_b200_solver* s, int a, int b, int c)
 {

@@ -788,6 +788,7 @@ bool build_tables(const Forest& f, const int mthbc[4], bool inflow, Tables& out,
         for (int a = f.lev_off[l]; a < f.lev_off[l + 1]; a += 64) pch.push_back({l, a, std::min(f.lev_off[l + 1], a + 64)});
     w.copy.resize(pch.size()); w.avg.resize(pch.size()); w.phys.resize(pch.size()); w.ti.resize(pch.size());
     out.sync.resize((size_t)np * SYNC_SLOTS);           // every slot is written by its patch's task
+    out.copy_nbr.resize(f.sphere() ? 0 : (size_t)np * 8);
     auto phys_sync = [&](int c) {
         const int a0 = pch[c].a, a1 = pch[c].b;
         // ---- setphysical: clawpack46_bc2_default with chains resolved per patch ----
@@ -858,19 +859,23 @@ bool build_tables(const Forest& f, const int mthbc[4], bool inflow, Tables& out,
         bool good = true;
         for (int ip = pch[c].a; ip < pch[c].b; ip++) {
             const PatchInfo& P = f.p[ip];
-            for (int fc = 0; fc < 4; fc++) {
-                if (P.face_type[fc] != NB_SAME) continue;
-                const int n = P.face_nbr[fc][0];
+            for (int region = 0; region < 8; region++) {
+                const int cr = region - 4;
+                const bool same = region < 4 ? P.face_type[region] == NB_SAME
+                                             : P.has_corner[cr] && P.corner_type[cr] == NB_SAME;
+                const int n = !same ? -1 : region < 4 ? P.face_nbr[region][0] : P.corner_nbr[cr];
+                if (!f.sphere()) out.copy_nbr[(size_t)ip * 8 + region] = n;
+                if (!same) continue;
                 const TableCtx::Aff A = T.same_map(P, f.p[n]);
-                good = good && copy_ok(fc, A);
-                vc.push_back(op(ip, n, fc, A));
-            }
-            for (int cr = 0; cr < 4; cr++) {
-                if (!P.has_corner[cr] || P.corner_type[cr] != NB_SAME) continue;
-                const int n = P.corner_nbr[cr];
-                const TableCtx::Aff A = T.same_map(P, f.p[n]);
-                good = good && copy_ok(4 + cr, A);
-                vc.push_back(op(ip, n, 4 + cr, A));
+                good = good && copy_ok(region, A) && n >= 0 && n < np;
+                if (f.sphere()) {
+                    vc.push_back(op(ip, n, region, A));
+                } else {
+                    // the kernel's shift: towards the neighbour by a patch width
+                    const int sx = region == 0 ? 1 : region == 1 ? -1 : region < 4 ? 0 : (cr & 1) ? -1 : 1;
+                    const int sy = region == 2 ? 1 : region == 3 ? -1 : region < 4 ? 0 : (cr & 2) ? -1 : 1;
+                    good = good && A.ii == 1 && A.jj == 1 && A.ij == 0 && A.ji == 0 && A.ci == sx * mx && A.cj == sy * my;
+                }
             }
             if (!P.on_cf) continue;
             for (int fc = 0; fc < 4; fc++) {

@@ -164,7 +164,8 @@ void make_partition(const Forest& f, int rank, int size, PartitionPlan& out);
 // Ghost-fill tables of a forest, flat in level order: level l's entries of table x are
 // x[x_off[l], x_off[l + 1]).
 struct Tables {
-    std::vector<FillOp> copy;        // copy2ghost(level): region ops of the level's patches
+    std::vector<FillOp> copy;        // copy2ghost(level) on the cubed sphere: region ops of the level's patches
+    std::vector<int> copy_nbr;       // copy2ghost on a brick: 8 same-size neighbours per patch (CopySeg)
     std::vector<FillOp> avg;         // average2ghost(level): level is the coarse level
     std::vector<InterpEnt> interp;   // interpolate2ghost(level): level is the coarse level
     std::vector<PhysEnt> phys;       // setphysical(level)

@@ -82,12 +82,17 @@ struct PhysEnt { int dst, src, neg, cst; };        // neg: bit m set => negate f
 
 // One table segment of a gather stage: entries e[0..n) from src into dst.
 template <class E> struct GatherSeg { double* dst; const double* src; const E* e; int n; };
+// copy2ghost of a brick: patches p0 .. p0 + np - 1 of array q take their ghost cells from their
+// same-size neighbours; nbr[8 p + region] is the neighbour's slot (regions as above), or -1.
+// Blocks of a brick are equally oriented, so a region's source cells are its own shifted by a
+// patch width.  (The cubed sphere, whose blocks turn, copies by FillOps.)
+struct CopySeg { double* q; int p0, np; };
 // average segments and copy segments of one ghost update in one launch (disjoint ghost
 // cells); area: per-patch cell areas (one ring more than q per patch) for the
 // area-weighted average of a manifold, or null for the plain mean.
 void launch_average_copy(const Dims& d, const GatherSeg<FillOp>& a0, const GatherSeg<FillOp>& a1,
-                         const GatherSeg<FillOp>& c0, const GatherSeg<FillOp>& c1, const double* area,
-                         cudaStream_t st);
+                         const GatherSeg<FillOp>& f0, const GatherSeg<FillOp>& f1, const CopySeg& c0,
+                         const CopySeg& c1, const int* nbr, const double* area, cudaStream_t st);
 void launch_restore_patches(const Dims& d, double* dst, const double* src, const int* slots, int n, cudaStream_t st);
 void launch_interp(const Dims& d, const GatherSeg<InterpEnt>& s0, const GatherSeg<InterpEnt>& s1, cudaStream_t st);
 void launch_phys(const Dims& d, const GatherSeg<PhysEnt>& s0, const GatherSeg<PhysEnt>& s1, const double* bcstate,
