@@ -394,7 +394,7 @@ struct RunSync {
 };
 constexpr int SYNC_MAX_MEQN = 8;
 template <class PS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 8)           // 32 registers: 1480 patches of 192 threads in one wave
 k_sync(double* __restrict__ q, const double* __restrict__ regs, const PatchDesc* __restrict__ desc,
        const int* __restrict__ src, int p0, int mx_, int my_, int mbc_, int meqn_, int nreg)
 {

@@ -163,6 +163,13 @@ struct WaveShallowRoe {
         if constexpr (sizeof(T) == 4) {
             // FP32: a1 + a3 = asdq_0, and the common factors of the components taken out
             const T a3 = asdq[0] - a1, s0 = v - a, s2 = v + a;
+            if (s0 < T(0) && s2 > T(0)) {                         // subcritical, the rule
+                const T m0 = s0 * a1, p2 = s2 * a3;
+                bm[0] = m0; bp[0] = p2;
+                bm[mu] = u * m0 + fmin(v, T(0)) * a2; bp[mu] = u * p2 + fmax(v, T(0)) * a2;
+                bm[mv] = m0 * s0; bp[mv] = p2 * s2;
+                return;
+            }
             const T m0 = fmin(s0, T(0)) * a1, m1 = fmin(v, T(0)) * a2, m2 = fmin(s2, T(0)) * a3;
             const T p0 = fmax(s0, T(0)) * a1, p1 = fmax(v, T(0)) * a2, p2 = fmax(s2, T(0)) * a3;
             bm[0] = m0 + m2; bp[0] = p0 + p2;
@@ -172,6 +179,15 @@ struct WaveShallowRoe {
         }
         const T a3 = (-((v - a) * asdq[0]) + asdq[mv]) / (T(2) * a);
         const T sb0 = v - a, sb1 = v, sb2 = v + a;
+        if (sb0 < T(0) && sb2 > T(0)) {
+            // subcritical, the rule: the outer waves go one way each (the products left out are
+            // zeros)
+            const T m1 = dmin1(sb1, T(0)) * a2, p1 = dmax1(sb1, T(0)) * a2;
+            bm[0] = sb0 * a1; bp[0] = sb2 * a3;
+            bm[mu] = sb0 * (a1 * u) + m1; bp[mu] = p1 + sb2 * (a3 * u);
+            bm[mv] = sb0 * (a1 * sb0); bp[mv] = sb2 * (a3 * sb2);
+            return;
+        }
         const T m0 = dmin1(sb0, T(0)), m1 = dmin1(sb1, T(0)), m2 = dmin1(sb2, T(0));
         const T p0 = dmax1(sb0, T(0)), p1 = dmax1(sb1, T(0)), p2 = dmax1(sb2, T(0));
         const T w0u = a1 * u, w0v = a1 * sb0, w2u = a3 * u, w2v = a3 * sb2;
