@@ -16,8 +16,9 @@
 //   cells   status, save_current_step, velocity scaling (b4step2), dt/dx/kappa
 //   faces   a and cq of every x and y interface, from q alone (the y sweep does not read the x
 //           sweep's results), indexed by the cell right of or above it
-//   update  per cell the four face fluxes with their transverse terms, formed from the
-//           records; q; CFL maximum; time-sync wave accumulation
+//   cross   the transverse terms of every face, from the records of the crossing sweep
+//   update  per cell the four face fluxes, formed from the records; q; CFL maximum; time-sync
+//           wave accumulation
 // Sums keep the order of clawpack46_step2.f, so FP64 results are the CPU path's bits; what is
 // dropped are additions of zeros.  At a corner of the cubed sphere (three blocks meet) the
 // faces phase runs sweep by sweep with that sweep's corner cells.
@@ -48,7 +49,8 @@ struct AdvGeom {
     static_assert(QBYTES % 16 == 0, "bulk copies move multiples of 16 bytes");
     static constexpr size_t OFF_A = QBYTES;                                  // aux [MAUX][NXY] double
     static constexpr size_t OFF_F = OFF_A + ABYTES;                          // a of x, y faces [2][NXY] double
-    static constexpr size_t OFF_C = OFF_F + 2 * QBYTES;                      // cq of x, y faces [2][NXY] TW
+    static constexpr size_t OFF_V = OFF_F + 2 * QBYTES;                      // transverse terms of x, y faces [2][NXY] double
+    static constexpr size_t OFF_C = OFF_V + 2 * QBYTES;                      // cq of x, y faces [2][NXY] TW
     static constexpr size_t OFF_R = OFF_C + 2 * (size_t)NXY * sizeof(TW);    // dt/(dx kappa), capacity only [NXY] TW
     static constexpr size_t OFF_Q = OFF_R + (MAUX == 3 ? (size_t)NXY * sizeof(TW) : 0);   // FP32 form: q in TW [NXY]
     static constexpr size_t OFF_RED = OFF_Q + (F32 ? (size_t)NXY * sizeof(TW) : 0);
@@ -88,6 +90,10 @@ struct AdvPatch {
     template <int IXY> __device__ __forceinline__ double* F() const
     {
         return reinterpret_cast<double*>(sm + G::OFF_F) + (IXY - 1) * NXY;
+    }
+    template <int IXY> __device__ __forceinline__ double* V() const
+    {
+        return reinterpret_cast<double*>(sm + G::OFF_V) + (IXY - 1) * NXY;
     }
     template <int IXY> __device__ __forceinline__ TW* C() const
     {
@@ -150,26 +156,33 @@ struct AdvPatch {
         const TW a = vel<IXY>(c) > 0.0 ? (TW)F<IXY>()[c] : TW(0);
         return M.order1() > 1 && M.order2() == 2 ? a - C<IXY>()[c] : a;
     }
-    // Fluxes fm, fp of the face left of (IXY 1) or below (IXY 2) cell c: own terms and the
-    // transverse terms of the crossing sweep from the upwind line, whose cell there is cu.
-    // pos, npos: the face's position along its sweep, and across it.
+    // Transverse terms of the face left of (IXY 1) or below (IXY 2) cell c: those of the crossing
+    // sweep from the upwind line, whose cell there is cu.  pos, npos: the face's position along
+    // its sweep, and across it.
     template <int IXY>
-    __device__ __forceinline__ void flux(int c, int pos, int npos, double& fm, double& fp) const
+    __device__ __forceinline__ void cross(int c, int pos, int npos) const
     {
-        constexpr int step = IXY == 1 ? 1 : NX, cross = IXY == 1 ? NX : 1, N = IXY == 1 ? NX : NY;
-        const double s = vel<IXY>(c), a = F<IXY>()[c];
-        const double h = G::F32 ? 0.5 * (double)C<IXY>()[c] : (double)(TW(0.5) * C<IXY>()[c]);
-        const bool god = pos <= N - 2;
-        fm = (god && s < 0.0 ? a : 0.0) + h;
-        fp = (god && s > 0.0 ? 0.0 - a : 0.0) + h;
-        if (M.order2() > 0 && (s > 0.0 ? pos - 1 >= 1 : s < 0.0 && god)) {
+        constexpr int step = IXY == 1 ? 1 : NX, side = IXY == 1 ? NX : 1, N = IXY == 1 ? NX : NY;
+        const double s = vel<IXY>(c);
+        double v = 0.0;
+        if (M.order2() > 0 && (s > 0.0 ? pos - 1 >= 1 : s < 0.0 && pos <= N - 2)) {
             const int cu = s > 0.0 ? c - step : c;
             const TW sv = (TW)s, r = TW(0.5) * ratio<3 - IXY>(cu);
-            double v = 0.0 - (double)(r * (sv * minus<3 - IXY>(cu + cross, npos + 1)));
+            v = 0.0 - (double)(r * (sv * minus<3 - IXY>(cu + side, npos + 1)));
             v = v - (double)(r * (sv * plus<3 - IXY>(cu)));
-            if (IXY == 1) { fm = fm + v; fp = fp + v; }
-            else { fm = v + fm; fp = v + fp; }
         }
+        V<IXY>()[c] = v;
+    }
+    // Fluxes fm, fp of that face.
+    template <int IXY>
+    __device__ __forceinline__ void flux(int c, int pos, double& fm, double& fp) const
+    {
+        constexpr int N = IXY == 1 ? NX : NY;
+        const double s = vel<IXY>(c), a = F<IXY>()[c], v = V<IXY>()[c];
+        const double h = G::F32 ? 0.5 * (double)C<IXY>()[c] : (double)(TW(0.5) * C<IXY>()[c]);
+        const bool god = pos <= N - 2;
+        fm = ((god && s < 0.0 ? a : 0.0) + h) + v;
+        fp = ((god && s > 0.0 ? 0.0 - a : 0.0) + h) + v;
     }
 };
 
@@ -277,6 +290,13 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
         faces(true, true);
     }
     __syncthreads();
+    // ---- transverse terms, once per face (two cells read each) --------------------------
+    for (int c = tid; c < NXY; c += NT) {
+        const int jc = c / NX, ic = c - jc * NX;
+        if (ic >= 1 && jc >= 1 && jc <= NY - 2) X.template cross<1>(c, ic, jc);
+        if (jc >= 1 && ic >= 1 && ic <= NX - 2) X.template cross<2>(c, jc, ic);
+    }
+    __syncthreads();
 
     // ---- time-sync wave accumulation (clawpack46_time_sync.f:163-226), FP64 ----
     if (sp->accumulate_waves) {
@@ -290,18 +310,18 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
             double fm, fp;
             if (it < MY) {
                 const int jc = MBC + it, c = jc * NX + MBC;
-                X.template flux<1>(c, MBC, jc, fm, fp);
+                X.template flux<1>(c, MBC, fm, fp);
                 add(0, G::R_FP0 + it, 0.0 - dtdyv * fp);
                 add(0, G::R_FM0 + it, dtdyv * fm);
-                X.template flux<1>(c + MX, MX + MBC, jc, fm, fp);
+                X.template flux<1>(c + MX, MX + MBC, fm, fp);
                 add(1, G::R_FP1 + it, 0.0 - dtdyv * fp);
                 add(1, G::R_FM1 + it, dtdyv * fm);
             } else {
                 const int i = it - MY, ic = MBC + i, c = MBC * NX + ic;
-                X.template flux<2>(c, MBC, ic, fm, fp);
+                X.template flux<2>(c, MBC, fm, fp);
                 add(2, G::R_GP0 + i, 0.0 - dtdxv * fp);
                 add(2, G::R_GM0 + i, dtdxv * fm);
-                X.template flux<2>(c + MY * NX, MY + MBC, ic, fm, fp);
+                X.template flux<2>(c + MY * NX, MY + MBC, fm, fp);
                 add(3, G::R_GP1 + i, 0.0 - dtdxv * fp);
                 add(3, G::R_GM1 + i, dtdxv * fm);
             }
@@ -316,12 +336,12 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
         if (ic <= NX - 2 && jc <= NY - 2) {
             double fr = 0.0, fl = 0.0, gt = 0.0, gb = 0.0, none;
             if (jc >= 1) {
-                X.template flux<1>(c + 1, ic + 1, jc, fr, none);
-                if (ic >= 1) X.template flux<1>(c, ic, jc, none, fl);
+                X.template flux<1>(c + 1, ic + 1, fr, none);
+                if (ic >= 1) X.template flux<1>(c, ic, none, fl);
             }
             if (ic >= 1) {
-                X.template flux<2>(c + NX, jc + 1, ic, gt, none);
-                if (jc >= 1) X.template flux<2>(c, jc, ic, none, gb);
+                X.template flux<2>(c + NX, jc + 1, gt, none);
+                if (jc >= 1) X.template flux<2>(c, jc, none, gb);
             }
             const double old = Q[c];
             double v = old;

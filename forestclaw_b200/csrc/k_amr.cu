@@ -796,10 +796,10 @@ void launch_average_copy(const Dims& d, const GatherSeg<FillOp>& a0, const Gathe
     const int nop = nblk(n, threads), grid = nop + c0.np + c1.np;
     if (grid <= 0) return;
     auto kern = area ? &k_average_copy<RunShape, true> : &k_average_copy<RunShape, false>;
-    if (!area && d.mx == d.my && d.mbc == 2) {
-        if (d.mx == 8) kern = &k_average_copy<FixedShape<8, 2>, false>;
-        else if (d.mx == 16) kern = &k_average_copy<FixedShape<16, 2>, false>;
-        else if (d.mx == 32) kern = &k_average_copy<FixedShape<32, 2>, false>;
+    if (d.mx == d.my && d.mbc == 2) {
+        if (d.mx == 8) kern = area ? &k_average_copy<FixedShape<8, 2>, true> : &k_average_copy<FixedShape<8, 2>, false>;
+        else if (d.mx == 16) kern = area ? &k_average_copy<FixedShape<16, 2>, true> : &k_average_copy<FixedShape<16, 2>, false>;
+        else if (d.mx == 32) kern = area ? &k_average_copy<FixedShape<32, 2>, true> : &k_average_copy<FixedShape<32, 2>, false>;
     }
     launch_k(kern, grid, threads, 0, st, a0, a1, f0, f1, c0, c1, nop, nbr, d.mx, d.my, d.mbc, d.meqn, area);
 }

@@ -10,7 +10,6 @@ const Step2Variant* step2_table_f32w_adv(int* n)
 {
     static const Step2Variant table[] = {
         FCB_ADV_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 448, 2, float, 4),
-        FCB_ADV_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 448, 3, float, 4),
         FCB_ADV_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 672, 2, float, 4),
         FCB_ADV_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 448, 2, float, 0),
         FCB_ADV_VARIANT(FC2D_B200_PREC_FP32WAVE, FC2D_B200_RP_ADVECTION, AdvPlane, 32, 672, 2, float, 0),
