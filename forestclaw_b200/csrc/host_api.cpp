@@ -216,6 +216,7 @@ struct fc2d_b200_solver {
     // and their stencil neighbours) is written by the interpolation into level l, so
     // the two (issued finer first) may share a launch; computed per forest
     unsigned char interp_chain[34] = {};
+    unsigned char phys_direct[34] = {};            // Tables::phys_direct of the current forest
     StepParams* tune_params = nullptr;             // autotuner: dt = 0 parameters (device)
     DevVec<RepopOp> repop_dev;                     // regrid repopulation ops
     DevVec<double> snap;                           // batch regrid: q of instances whose forest is unchanged
@@ -478,6 +479,7 @@ static int upload_desc_and_tables(fc2d_b200_solver* s)
         r.phys_off = T.phys_off[l]; r.phys_n = T.phys_off[l + 1] - T.phys_off[l];
         r.ti_off = T.ti_off[l]; r.ti_n = T.ti_off[l + 1] - T.ti_off[l];
     }
+    std::memcpy(s->phys_direct, T.phys_direct, sizeof(s->phys_direct));
     const std::vector<InterpEnt>& interp = T.interp;
     {
         TableArena& A = s->arena;
@@ -691,8 +693,11 @@ static GatherSeg<E> seg(const E* table, int off, int n, double* dst, const doubl
 // average2ghost of coarse levels [a, b] and copy2ghost of levels [ca, cb] (with level c
 // of the time-interpolated copy for both) in one launch: the two stages write disjoint
 // ghost cells and read interior cells only, so their order does not matter
-static void average_copy_range(fc2d_b200_solver* s, int a, int b, int ca, int cb, int c)
+// (phys: and the physical BCs of levels [ca, cb], whose sources are interior cells)
+static void average_copy_range(fc2d_b200_solver* s, int a, int b, int ca, int cb, int c, bool phys)
 {
+    GatherSeg<PhysEnt> ph{nullptr, nullptr, nullptr, 0};
+
     GatherSeg<FillOp> a0{nullptr, nullptr, nullptr, 0}, a1 = a0, f0 = a0, f1 = a0;
     CopySeg c0{nullptr, 0, 0}, c1 = c0;
     const int* lev_off = s->forest.lev_off;
@@ -705,16 +710,20 @@ static void average_copy_range(fc2d_b200_solver* s, int a, int b, int ca, int cb
     if (lrange(ca, cb)) {
         const int off = s->lr[ca].copy_off, n = s->lr[cb].copy_off + s->lr[cb].copy_n - off;
         if (n > 0) f0 = seg(s->t_copy.p, off, n, s->q, s->q);
+        if (phys) {
+            const int po = s->lr[ca].phys_off, pn = s->lr[cb].phys_off + s->lr[cb].phys_n - po;
+            if (pn > 0) ph = seg(s->t_phys.p, po, pn, s->q, s->q);
+        }
         if (!s->sphere && lev_off[cb + 1] - lev_off[ca] > 1) c0 = CopySeg{s->q, lev_off[ca], lev_off[cb + 1] - lev_off[ca]};
     }
     if (c >= 0 && c <= 32) {
         if (s->lr[c].copy_n > 0) f1 = seg(s->t_copy.p, s->lr[c].copy_off, s->lr[c].copy_n, s->qinterp, s->qinterp);
         if (!s->sphere && lev_off[c + 1] - lev_off[c] > 1) c1 = CopySeg{s->qinterp, lev_off[c], lev_off[c + 1] - lev_off[c]};
     }
-    if (a0.n + a1.n + f0.n + f1.n + c0.np + c1.np <= 0) return;
+    if (a0.n + a1.n + f0.n + f1.n + c0.np + c1.np + ph.n <= 0) return;
     (void)flush_pending(s);
     if (s->fill) s->total_launches++;
-    if (s->emit) launch_average_copy(s->d, a0, a1, f0, f1, c0, c1, s->t_nbr.p, s->area, s->st);
+    if (s->emit) launch_average_copy(s->d, a0, a1, f0, f1, c0, c1, s->t_nbr.p, s->area, ph, s->bc_dev, s->st);
 }
 static void phys_range(fc2d_b200_solver* s, int a, int b, int c)
 {
@@ -850,7 +859,13 @@ static void ghost_update(fc2d_b200_solver* s, int minlevel, int maxlevel, int ti
         for (int l = std::max(minlevel, 0); l <= std::min(maxlevel, 63); l++) s->phys_ok[l] = 1;
     const int mincoarse = minlevel, maxcoarse = maxlevel - 1;
     const int ti = time_interp ? mincoarse - 1 : -1;      // level of the time-interpolated copy
-    average_copy_range(s, mincoarse, maxcoarse, minlevel, maxlevel, ti);
+    if (minlevel == maxlevel && ti < 0 && minlevel >= 0 && minlevel <= 32 && s->phys_direct[minlevel]) {
+        // one level: nothing to average or interpolate, and its physical BCs read what the copy
+        // stage reads
+        average_copy_range(s, mincoarse, maxcoarse, minlevel, maxlevel, ti, true);
+        return;
+    }
+    average_copy_range(s, mincoarse, maxcoarse, minlevel, maxlevel, ti, false);
     phys_range(s, mincoarse, maxcoarse, ti);
     interpolate_levels(s, mincoarse, maxcoarse, time_interp);
     // the reference applies the physical BC to the fine levels [mincoarse+1, maxlevel],

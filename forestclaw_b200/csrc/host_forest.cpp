@@ -789,8 +789,25 @@ bool build_tables(const Forest& f, const int mthbc[4], bool inflow, Tables& out,
     w.copy.resize(pch.size()); w.avg.resize(pch.size()); w.phys.resize(pch.size()); w.ti.resize(pch.size());
     out.sync.resize((size_t)np * SYNC_SLOTS);           // every slot is written by its patch's task
     out.copy_nbr.resize(f.sphere() ? 0 : (size_t)np * 8);
+    // A physical-BC source that is a ghost cell beside a same-size neighbour becomes the
+    // neighbour's interior cell copy2ghost takes it from (on a brick): the same value, and no
+    // dependence on the copy stage.  Whether src is an interior cell then.
+    auto interior_source = [&](int ip, int base, int& src) {
+        const PatchInfo& P = f.p[ip];
+        const int i = (src - base) % T.nx, j = (src - base) / T.nx;      // padded, 0-based
+        const int sx = i < mbc ? -1 : i >= mx + mbc ? 1 : 0, sy = j < mbc ? -1 : j >= my + mbc ? 1 : 0;
+        if (sx == 0 && sy == 0) return true;
+        if (f.sphere()) return false;
+        const int fc = sy == 0 ? (sx > 0) : 2 + (sy > 0), cr = (sx > 0) + 2 * (sy > 0);
+        const bool face = sx == 0 || sy == 0;
+        if (face ? P.face_type[fc] != NB_SAME : !(P.has_corner[cr] && P.corner_type[cr] == NB_SAME)) return false;
+        src = T.cell(face ? P.face_nbr[fc][0] : P.corner_nbr[cr], i - sx * mx + 1 - mbc, j - sy * my + 1 - mbc);
+        return true;
+    };
+    w.direct.assign(pch.size(), 1);
     auto phys_sync = [&](int c) {
         const int a0 = pch[c].a, a1 = pch[c].b;
+        bool direct = true;
         // ---- setphysical: clawpack46_bc2_default with chains resolved per patch ----
         {
             std::vector<int> wsrc(nxy, -1), wneg(nxy, 0), wconst(nxy, 0);
@@ -830,9 +847,14 @@ bool build_tables(const Forest& f, const int mthbc[4], bool inflow, Tables& out,
                 if (bc[2] == 3) for (int jbc = 1; jbc <= mbc; jbc++) for (int i = 1 - mbc; i <= mx + mbc; i++) put(i, 1 - jbc, i, jbc, NEG3);
                 if (bc[3] == 1) for (int jbc = 1; jbc <= mbc; jbc++) for (int i = 1 - mbc; i <= mx + mbc; i++) put(i, my + jbc, i, my, 0);
                 if (bc[3] == 3) for (int jbc = 1; jbc <= mbc; jbc++) for (int i = 1 - mbc; i <= mx + mbc; i++) put(i, my + jbc, i, my + 1 - jbc, NEG3);
-                for (int dst : order) w.phys[c].push_back({dst, wsrc[dst - base], wneg[dst - base], wconst[dst - base]});
+                for (int dst : order) {
+                    int src = wsrc[dst - base];
+                    if (!wconst[dst - base] && !interior_source(ip, base, src)) direct = false;
+                    w.phys[c].push_back({dst, src, wneg[dst - base], wconst[dst - base]});
+                }
             }
         }
+        w.direct[c] = direct;
         // ---- time interpolation patches ----
         for (int ip = a0; ip < a1; ip++) if (f.p[ip].has_fine_nbr) w.ti[c].push_back(ip);
         // ---- time-sync sources: per face and half of it the neighbour whose registers
@@ -1023,7 +1045,8 @@ bool build_tables(const Forest& f, const int mthbc[4], bool inflow, Tables& out,
         out.phys_off[l] = (int)oph[c];
         out.ti_off[l] = (int)oti[c];
         out.interp_off[l] = (int)oi[ci];
-        while (c < npch && pch[c].l == l) c++;
+        out.phys_direct[l] = 1;
+        while (c < npch && pch[c].l == l) out.phys_direct[l] &= w.direct[c++];
         while (ci < nchunk && chunks[ci].l == l) ci++;
     }
     // (no clear first: a vector that shrinks or keeps its size is not refilled with zeros)

@@ -172,6 +172,7 @@ struct Tables {
     std::vector<int> ti;             // patches with fine-grid neighbours (fclaw2d_timeinterp)
     std::vector<int> sync;           // time-sync sources, SYNC_SLOTS per patch (launch_sync)
     int copy_off[34], avg_off[34], interp_off[34], phys_off[34], ti_off[34];
+    unsigned char phys_direct[34];   // the level's physical-BC sources are interior cells all
 };
 
 // Buffers build_tables keeps between calls (their pages stay mapped from one regrid
@@ -184,6 +185,7 @@ struct TableWork {
     std::vector<std::vector<FillOp>> copy, avg;            // region ops per chunk of patches
     std::vector<std::vector<PhysEnt>> phys;                // physical-BC entries per chunk of patches
     std::vector<std::vector<int>> ti;                      // time-interpolation patches per chunk
+    std::vector<unsigned char> direct;                     // physical-BC sources all interior, per chunk
     std::vector<std::vector<InterpOp>> iops;               // interpolation ops per coarse level, by fine patch
     std::vector<std::vector<int>> iop_first;               // per coarse level: CSR offsets over its fine patches
     std::vector<std::vector<InterpEnt>> interp;            // interpolation entries per task

@@ -222,26 +222,44 @@ __device__ __forceinline__ void copy_patch(const S& P, double* __restrict__ q, i
     }
 }
 
+__device__ __forceinline__ void phys_at(const GatherSeg<PhysEnt>& s0, const GatherSeg<PhysEnt>& s1, long t, int nxy,
+                                        int meqn, const double* __restrict__ bcstate)
+{
+    GatherSeg<PhysEnt> g;
+    int e, m;
+    if (!seg_item(s0, s1, meqn, t, g, e, m)) return;
+    double* __restrict__ q = g.dst;                 // in place: sources are cells of the same array
+    const PhysEnt c = g.e[e];
+    const double v = c.cst ? bcstate[m] : q[c.src + m * nxy];
+    q[c.dst + m * nxy] = ((c.neg >> m) & 1) ? -v : v;
+}
 // The average and copy stages of one ghost update in one launch: averaging writes
 // the ghost cells a coarse patch has beside finer neighbours, copying those beside
 // same-size neighbours (disjoint cells), and both read interior cells only, which
 // neither writes.  The first nop CTAs run region ops, one thread per (op, cell) with
 // mbc * max(mx, my) threads per op (a face's cells; a corner uses mbc * mbc of them): the
-// average segments, then the cubed sphere's copy segments.  The others copy, one CTA per patch
-// of a brick.  (Copies as region ops too took 16.7 us for 4096 16x16 patches of three fields:
+// average segments, then the cubed sphere's copy segments.  The next ncopy CTAs copy, one per
+// patch of a brick; the rest apply physical BCs whose sources are interior cells (all of a
+// uniform forest's: a launch of 3 us saved per step).  (Copies as region ops too took 16.7 us for 4096 16x16 patches of three fields:
 // 8 x 32 threads per patch for its 144 cells, each unpacking its op and mapping its cell.)
 // AREA: the area-weighted average of a manifold (cell areas in `area`).
 template <class S, bool AREA>
 __global__ void __launch_bounds__(288)
 k_average_copy(GatherSeg<FillOp> a0, GatherSeg<FillOp> a1, GatherSeg<FillOp> f0, GatherSeg<FillOp> f1, CopySeg c0,
                CopySeg c1, int nop, const int* __restrict__ nbr, int mx, int my, int mbc, int meqn,
-               const double* __restrict__ area)
+               const double* __restrict__ area, GatherSeg<PhysEnt> ph, const double* __restrict__ bcstate)
 {
     grid_dependency_wait();       // programmatic launch: the previous grid's writes are visible
     grid_launch_dependents();
     const S P(mx, my, mbc);
     if ((int)blockIdx.x >= nop) {
         const int b = (int)blockIdx.x - nop;
+        if (b >= c0.np + c1.np) {
+            const GatherSeg<PhysEnt> none{nullptr, nullptr, nullptr, 0};
+            phys_at(ph, none, (long)(b - c0.np - c1.np) * blockDim.x + threadIdx.x,
+                    (P.mx + 2 * P.mbc) * (P.my + 2 * P.mbc), meqn, bcstate);
+            return;
+        }
         const bool second = b >= c0.np;
         copy_patch(P, second ? c1.q : c0.q, second ? c1.p0 + b - c0.np : c0.p0 + b, nbr, meqn);
         return;
@@ -297,17 +315,6 @@ __global__ void k_interp(GatherSeg<InterpEnt> s0, GatherSeg<InterpEnt> s1, int n
     interp_at(s0, s1, flat_index(), nx, nxy, meqn);
 }
 
-__device__ __forceinline__ void phys_at(const GatherSeg<PhysEnt>& s0, const GatherSeg<PhysEnt>& s1, long t, int nxy,
-                                        int meqn, const double* __restrict__ bcstate)
-{
-    GatherSeg<PhysEnt> g;
-    int e, m;
-    if (!seg_item(s0, s1, meqn, t, g, e, m)) return;
-    double* __restrict__ q = g.dst;                 // in place: sources are cells of the same array
-    const PhysEnt c = g.e[e];
-    const double v = c.cst ? bcstate[m] : q[c.src + m * nxy];
-    q[c.dst + m * nxy] = ((c.neg >> m) & 1) ? -v : v;
-}
 __global__ void k_phys(GatherSeg<PhysEnt> s0, GatherSeg<PhysEnt> s1, int nxy, int meqn,
                        const double* __restrict__ bcstate)
 {
@@ -788,12 +795,13 @@ void launch_restore_patches(const Dims& d, double* dst, const double* src, const
 
 void launch_average_copy(const Dims& d, const GatherSeg<FillOp>& a0, const GatherSeg<FillOp>& a1,
                          const GatherSeg<FillOp>& f0, const GatherSeg<FillOp>& f1, const CopySeg& c0,
-                         const CopySeg& c1, const int* nbr, const double* area, cudaStream_t st)
+                         const CopySeg& c1, const int* nbr, const double* area, const GatherSeg<PhysEnt>& ph,
+                         const double* bcstate, cudaStream_t st)
 {
     const long n = ((long)a0.n + a1.n + f0.n + f1.n) * d.mbc * (d.mx > d.my ? d.mx : d.my);
     const int cells = d.nxy() - d.mx * d.my;
     const int threads = cells < 288 ? (cells + 31) / 32 * 32 : 288;
-    const int nop = nblk(n, threads), grid = nop + c0.np + c1.np;
+    const int nop = nblk(n, threads), grid = nop + c0.np + c1.np + nblk((long)ph.n * d.meqn, threads);
     if (grid <= 0) return;
     auto kern = area ? &k_average_copy<RunShape, true> : &k_average_copy<RunShape, false>;
     if (d.mx == d.my && d.mbc == 2) {
@@ -801,7 +809,8 @@ void launch_average_copy(const Dims& d, const GatherSeg<FillOp>& a0, const Gathe
         else if (d.mx == 16) kern = area ? &k_average_copy<FixedShape<16, 2>, true> : &k_average_copy<FixedShape<16, 2>, false>;
         else if (d.mx == 32) kern = area ? &k_average_copy<FixedShape<32, 2>, true> : &k_average_copy<FixedShape<32, 2>, false>;
     }
-    launch_k(kern, grid, threads, 0, st, a0, a1, f0, f1, c0, c1, nop, nbr, d.mx, d.my, d.mbc, d.meqn, area);
+    launch_k(kern, grid, threads, 0, st, a0, a1, f0, f1, c0, c1, nop, nbr, d.mx, d.my, d.mbc, d.meqn, area,
+             ph, bcstate);
 }
 void launch_interp(const Dims& d, const GatherSeg<InterpEnt>& s0, const GatherSeg<InterpEnt>& s1, cudaStream_t st)
 {
