@@ -254,6 +254,7 @@ struct fc2d_b200_solver {
     char* block_dev = nullptr;
     char* block_host = nullptr;
     char* result_host = nullptr;
+    bool result_due = false;                       // the next averaging launch brings the result down
     unsigned long long* cfl_dev = nullptr;
     unsigned int* status_dev = nullptr;            // device status word (STATUS_* bits)
     double* mass_dev = nullptr;
@@ -690,6 +691,11 @@ static GatherSeg<E> seg(const E* table, int off, int n, double* dst, const doubl
 {
     return GatherSeg<E>{dst, src, table + off, n};
 }
+// Bytes of the step block's result (status word and CFL maxima).
+static size_t result_bytes(const fc2d_b200_solver* s)
+{
+    return (fc2d_b200_solver::BLK_CFL + 8 * (size_t)s->ncfl + 15) / 16 * 16;
+}
 // average2ghost of coarse levels [a, b] and copy2ghost of levels [ca, cb] (with level c
 // of the time-interpolated copy for both) in one launch: the two stages write disjoint
 // ghost cells and read interior cells only, so their order does not matter
@@ -723,7 +729,13 @@ static void average_copy_range(fc2d_b200_solver* s, int a, int b, int ca, int cb
     if (a0.n + a1.n + f0.n + f1.n + c0.np + c1.np + ph.n <= 0) return;
     (void)flush_pending(s);
     if (s->fill) s->total_launches++;
-    if (s->emit) launch_average_copy(s->d, a0, a1, f0, f1, c0, c1, s->t_nbr.p, s->area, ph, s->bc_dev, s->st);
+    ResultCopy res{nullptr, nullptr, 0};
+    if (s->result_due) {
+        res = ResultCopy{reinterpret_cast<uint4*>(s->result_host), reinterpret_cast<const uint4*>(s->block_dev),
+                         (int)(result_bytes(s) / 16)};
+        s->result_due = false;
+    }
+    if (s->emit) launch_average_copy(s->d, a0, a1, f0, f1, c0, c1, s->t_nbr.p, s->area, ph, s->bc_dev, res, s->st);
 }
 static void phys_range(fc2d_b200_solver* s, int a, int b, int c)
 {
@@ -1401,10 +1413,6 @@ static int begin_cfl(fc2d_b200_solver* s)
     return 0;
 }
 // The status word and CFL maxima of the work on the stream, to result_host.
-static size_t result_bytes(const fc2d_b200_solver* s)
-{
-    return (fc2d_b200_solver::BLK_CFL + 8 * (size_t)s->ncfl + 15) / 16 * 16;
-}
 static cudaError_t fetch_result(fc2d_b200_solver* s)
 {
     return cudaMemcpyAsync(s->result_host, s->block_dev, result_bytes(s), cudaMemcpyDeviceToHost, s->st);
@@ -1633,6 +1641,8 @@ static int traverse_advance(fc2d_b200_solver* s, double t, double dt)
             }
         }
     }
+    // the updates of the advance end here, and with them its status word and CFL maxima
+    s->result_due = !s->part;
     ghost_update(s, minlevel, maxlevel, 0);
     if (o.time_sync) time_sync(s, minlevel, maxlevel);
     return flush_pending(s);
@@ -1651,6 +1661,7 @@ static int advance_launch(fc2d_b200_solver_t* s, double t, double dt)
     // pass 1: host traversal filling the per-launch parameters and statistics
     s->emit = false; s->fill = true;
     int rc = traverse_advance(s, t, dt);
+    s->result_due = false;
     if (rc) { s->emit = true; return rc; }
     s->step_host_ms = wall_ms() - h0;
     cudaEvent_t* ev = s->step_ev[s->step_pair];
@@ -1666,8 +1677,10 @@ static int advance_launch(fc2d_b200_solver_t* s, double t, double dt)
         launch_step_begin(s->block_dev, s->block_host,
                           (fc2d_b200_solver::BLK_PARAMS + sizeof(StepParams) * nupd + 15) / 16 * 16, s->st);
         int r = traverse_advance(s, t, dt);
+        const bool due = s->result_due || s->part;      // not gone out with the last ghost update
+        s->result_due = false;
         if (r) return r;
-        launch_step_end(s->result_host, s->block_dev, result_bytes(s), s->st);
+        if (due) launch_step_end(s->result_host, s->block_dev, result_bytes(s), s->st);
         return 0;
     };
     // pass 2: the launches, captured once per forest into a CUDA graph and replayed

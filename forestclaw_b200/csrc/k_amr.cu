@@ -239,21 +239,27 @@ __device__ __forceinline__ void phys_at(const GatherSeg<PhysEnt>& s0, const Gath
 // neither writes.  The first nop CTAs run region ops, one thread per (op, cell) with
 // mbc * max(mx, my) threads per op (a face's cells; a corner uses mbc * mbc of them): the
 // average segments, then the cubed sphere's copy segments.  The next ncopy CTAs copy, one per
-// patch of a brick; the rest apply physical BCs whose sources are interior cells (all of a
-// uniform forest's: a launch of 3 us saved per step).  (Copies as region ops too took 16.7 us for 4096 16x16 patches of three fields:
-// 8 x 32 threads per patch for its 144 cells, each unpacking its op and mapping its cell.)
+// patch of a brick; the next apply physical BCs whose sources are interior cells (all of a
+// uniform forest's: a launch of 3 us saved per step).  One more CTA may bring down the step's
+// result (ResultCopy), which is complete once the step's updates are: another launch saved.
+// (Copies as region ops too took 16.7 us for 4096 16x16 patches of three fields: 8 x 32 threads
+// per patch for its 144 cells, each unpacking its op and mapping its cell.)
 // AREA: the area-weighted average of a manifold (cell areas in `area`).
 template <class S, bool AREA>
 __global__ void __launch_bounds__(288)
 k_average_copy(GatherSeg<FillOp> a0, GatherSeg<FillOp> a1, GatherSeg<FillOp> f0, GatherSeg<FillOp> f1, CopySeg c0,
                CopySeg c1, int nop, const int* __restrict__ nbr, int mx, int my, int mbc, int meqn,
-               const double* __restrict__ area, GatherSeg<PhysEnt> ph, const double* __restrict__ bcstate)
+               const double* __restrict__ area, GatherSeg<PhysEnt> ph, const double* __restrict__ bcstate, ResultCopy res)
 {
     grid_dependency_wait();       // programmatic launch: the previous grid's writes are visible
     grid_launch_dependents();
     const S P(mx, my, mbc);
     if ((int)blockIdx.x >= nop) {
         const int b = (int)blockIdx.x - nop;
+        if (res.n > 0 && blockIdx.x == gridDim.x - 1) {
+            for (int k = threadIdx.x; k < res.n; k += blockDim.x) res.to[k] = res.from[k];
+            return;
+        }
         if (b >= c0.np + c1.np) {
             const GatherSeg<PhysEnt> none{nullptr, nullptr, nullptr, 0};
             phys_at(ph, none, (long)(b - c0.np - c1.np) * blockDim.x + threadIdx.x,
@@ -796,12 +802,12 @@ void launch_restore_patches(const Dims& d, double* dst, const double* src, const
 void launch_average_copy(const Dims& d, const GatherSeg<FillOp>& a0, const GatherSeg<FillOp>& a1,
                          const GatherSeg<FillOp>& f0, const GatherSeg<FillOp>& f1, const CopySeg& c0,
                          const CopySeg& c1, const int* nbr, const double* area, const GatherSeg<PhysEnt>& ph,
-                         const double* bcstate, cudaStream_t st)
+                         const double* bcstate, const ResultCopy& res, cudaStream_t st)
 {
     const long n = ((long)a0.n + a1.n + f0.n + f1.n) * d.mbc * (d.mx > d.my ? d.mx : d.my);
     const int cells = d.nxy() - d.mx * d.my;
     const int threads = cells < 288 ? (cells + 31) / 32 * 32 : 288;
-    const int nop = nblk(n, threads), grid = nop + c0.np + c1.np + nblk((long)ph.n * d.meqn, threads);
+    const int nop = nblk(n, threads), grid = nop + c0.np + c1.np + nblk((long)ph.n * d.meqn, threads) + (res.n > 0);
     if (grid <= 0) return;
     auto kern = area ? &k_average_copy<RunShape, true> : &k_average_copy<RunShape, false>;
     if (d.mx == d.my && d.mbc == 2) {
@@ -810,7 +816,7 @@ void launch_average_copy(const Dims& d, const GatherSeg<FillOp>& a0, const Gathe
         else if (d.mx == 32) kern = area ? &k_average_copy<FixedShape<32, 2>, true> : &k_average_copy<FixedShape<32, 2>, false>;
     }
     launch_k(kern, grid, threads, 0, st, a0, a1, f0, f1, c0, c1, nop, nbr, d.mx, d.my, d.mbc, d.meqn, area,
-             ph, bcstate);
+             ph, bcstate, res);
 }
 void launch_interp(const Dims& d, const GatherSeg<InterpEnt>& s0, const GatherSeg<InterpEnt>& s1, cudaStream_t st)
 {

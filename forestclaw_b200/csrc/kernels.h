@@ -90,11 +90,12 @@ struct CopySeg { double* q; int p0, np; };
 // average segments and copy segments of one ghost update in one launch (disjoint ghost
 // cells); area: per-patch cell areas (one ring more than q per patch) for the
 // area-weighted average of a manifold, or null for the plain mean.  ph: physical-BC entries that
-// read interior cells only (or n = 0).
+// read interior cells only (or n = 0).  res: a result copied down by one more CTA (or n = 0).
+struct ResultCopy { uint4* to; const uint4* from; int n; };
 void launch_average_copy(const Dims& d, const GatherSeg<FillOp>& a0, const GatherSeg<FillOp>& a1,
                          const GatherSeg<FillOp>& f0, const GatherSeg<FillOp>& f1, const CopySeg& c0,
                          const CopySeg& c1, const int* nbr, const double* area, const GatherSeg<PhysEnt>& ph,
-                         const double* bcstate, cudaStream_t st);
+                         const double* bcstate, const ResultCopy& res, cudaStream_t st);
 void launch_restore_patches(const Dims& d, double* dst, const double* src, const int* slots, int n, cudaStream_t st);
 void launch_interp(const Dims& d, const GatherSeg<InterpEnt>& s0, const GatherSeg<InterpEnt>& s1, cudaStream_t st);
 void launch_phys(const Dims& d, const GatherSeg<PhysEnt>& s0, const GatherSeg<PhysEnt>& s1, const double* bcstate,
