@@ -36,7 +36,14 @@
 //   * the limiter reads the upwind neighbour's wave only;
 //   * LIM > 0 fixes the method at compile time (second order, second-order transverse terms,
 //     that limiter on every wave); LIM = 0 reads it from the launch's parameters.
-// Measured against the kernel it replaces: see the table at the launchers (run_wave_variant).
+// Updates of one coarse step, one B200, against the kernels it replaced (us, ncu, warm):
+//   radial dam levels 3-7, 1960 patches 16x16    FP32-wave  832 ->  620   FP64 1957 -> 1005
+//   radial dam uniform, 4096 patches 16x16       FP32-wave  108 ->   87
+//   radial dam uniform, 1536 patches 8x8, LIM 0                           FP64   72 ->   27
+//   tsunami batch, 8180 patches 8x8              FP32-wave 1230 ->  592
+//   tsunami uniform, 1024 patches 16x16                                   FP64  156 ->   71
+//   shock-bubble levels 4-7, 1784 patches 16x16  FP32-wave 1139 ->  473
+//   shock-bubble uniform, 512 patches 16x16                               FP64  172 ->   91
 //
 // Index conventions: padded 0-based cell (ic, jc), ic = i + mbc - 1 for the Fortran index i.
 // Interface ic sits between cells ic-1 and ic.  x interface k: row jc = 1 + k / (NX-1),
@@ -159,11 +166,15 @@ struct WavePatch {
     template <int IXY>
     __device__ __forceinline__ int normal(int k, int cL, int cR, double seed, St& st, TW* s) const
     {
-        TW qL[MEQN], qR[MEQN], aL[MA], aR[MA], w[MWAVES][MEQN];
+        TW qL[MEQN], qR[MEQN], dq[MEQN], aL[MA], aR[MA], da[MA], w[MWAVES][MEQN];
         for (int m = 0; m < MEQN; m++) { qL[m] = qc(m, cL); qR[m] = qc(m, cR); }
         for (int a = 0; a < MAUX; a++) { aL[a] = (TW)A()[a * NXY + cL]; aR[a] = (TW)A()[a * NXY + cR]; }
+        // FP64 differences, for the solver that forms its flux difference from them (the
+        // difference of two FP32 states keeps their rounding)
+        for (int m = 0; m < MEQN; m++) dq[m] = (TW)(Q()[m * NXY + cR] - Q()[m * NXY + cL]);
+        for (int a = 0; a < MAUX; a++) da[a] = (TW)(A()[a * NXY + cR] - A()[a * NXY + cL]);
         const TW* pc = C() + (F32 ? MEQN * NXY : 0);
-        const int it = RP::template normal<IXY>(qL, qR, aL, aR, Cell{pc + cL}, Cell{pc + cR}, P, seed, st, w, s);
+        const int it = RP::template normal<IXY>(qL, qR, dq, aL, aR, da, Cell{pc + cL}, Cell{pc + cR}, P, seed, st, w, s);
 #pragma unroll
         for (int mw = 0; mw < MWAVES; mw++)
 #pragma unroll

@@ -73,10 +73,10 @@ struct WaveShallowRoe {
     }
     template <typename T> struct State { T a1, a2, a3, u, v, a, am[3]; };
     template <int IXY, typename T, class C>
-    __device__ static int normal(const T* qL, const T* qR, const T* aL, const T* aR, C cL, C cR, const WavePar<T>& P,
-                                 double, State<T>& st, T w[3][3], T* s)
+    __device__ static int normal(const T* qL, const T* qR, const T* dq, const T* aL, const T* aR, const T* da, C cL, C cR,
+                                 const WavePar<T>& P, double, State<T>& st, T w[3][3], T* s)
     {
-        (void)aL; (void)aR;
+        (void)dq; (void)aL; (void)aR; (void)da;
         constexpr int mu = Dir<IXY>::mu, mv = Dir<IXY>::mv;
         constexpr int NN = IXY == 1 ? P_N1 : P_N2, NT = IXY == 1 ? P_N2 : P_N1;
         // :91-99
@@ -160,23 +160,6 @@ struct WaveShallowRoe {
         const T u = e.u, v = e.v, a = e.a;
         const T a1 = ((v + a) * asdq[0] - asdq[mv]) / (T(2) * a);
         const T a2 = asdq[mu] - u * asdq[0];
-        if constexpr (sizeof(T) == 4) {
-            // FP32: a1 + a3 = asdq_0, and the common factors of the components taken out
-            const T a3 = asdq[0] - a1, s0 = v - a, s2 = v + a;
-            if (s0 < T(0) && s2 > T(0)) {                         // subcritical, the rule
-                const T m0 = s0 * a1, p2 = s2 * a3;
-                bm[0] = m0; bp[0] = p2;
-                bm[mu] = u * m0 + fmin(v, T(0)) * a2; bp[mu] = u * p2 + fmax(v, T(0)) * a2;
-                bm[mv] = m0 * s0; bp[mv] = p2 * s2;
-                return;
-            }
-            const T m0 = fmin(s0, T(0)) * a1, m1 = fmin(v, T(0)) * a2, m2 = fmin(s2, T(0)) * a3;
-            const T p0 = fmax(s0, T(0)) * a1, p1 = fmax(v, T(0)) * a2, p2 = fmax(s2, T(0)) * a3;
-            bm[0] = m0 + m2; bp[0] = p0 + p2;
-            bm[mu] = u * bm[0] + m1; bp[mu] = u * bp[0] + p1;
-            bm[mv] = m0 * s0 + m2 * s2; bp[mv] = p0 * s0 + p2 * s2;
-            return;
-        }
         const T a3 = (-((v - a) * asdq[0]) + asdq[mv]) / (T(2) * a);
         const T sb0 = v - a, sb1 = v, sb2 = v + a;
         if (sb0 < T(0) && sb2 > T(0)) {
@@ -243,21 +226,29 @@ struct WaveShallowFWave {
     // t1, t2, t3: speeds of the transverse solve; dry: both cells below the tolerance
     template <typename T> struct State { T b1, b2, b3, s1, s3, vL, vR, t1, t2, t3; bool dry; };
     template <int IXY, typename T, class C>
-    __device__ static int normal(const T* qL, const T* qR, const T* aL, const T* aR, C cL, C cR, const WavePar<T>& P,
-                                 double, State<T>& st, T w[3][3], T* s)
+    __device__ static int normal(const T* qL, const T* qR, const T* dq, const T* aL, const T* aR, const T* da, C cL, C cR,
+                                 const WavePar<T>& P, double, State<T>& st, T w[3][3], T* s)
     {
         constexpr int UN = IXY == 1 ? P_U1 : P_U2, UT = IXY == 1 ? P_U2 : P_U1, EN = IXY == 1 ? P_E1 : P_E2;
         const T grav = P.grav;
         const T hL = qL[0], hR = qR[0];
         const T uR = cR(UN), vR = cR(UT), uL = cL(UN), vL = cL(UT);
-        const T phiR = T(0.5) * grav * (hR * hR) + cR(EN);
-        const T phiL = T(0.5) * grav * (hL * hL) + cL(EN);
         const T gL = cL(P_C), gR = cR(P_C);
         const T uhat = (gL * uL + gR * uR) / (gR + gL);
         const T chat = sqrt(grav * T(0.5) * (hR + hL));
         const T hbar = T(0.5) * (hR + hL);
-        const T fd1 = (hR * uR) - (hL * uL);
-        const T fd2 = phiR - phiL + grav * hbar * (aR[0] - aL[0]);
+        T fd1, fd2;
+        if constexpr (sizeof(T) == 4) {
+            // FP32: from the FP64 differences; g/2 (hR^2 - hL^2) is g hbar (hR - hL), so still
+            // water over any bottom balances to the rounding of h + b
+            fd1 = dq[IXY];
+            fd2 = grav * hbar * (dq[0] + da[0]) + (cR(EN) - cL(EN));
+        } else {
+            const T phiR = T(0.5) * grav * (hR * hR) + cR(EN);
+            const T phiL = T(0.5) * grav * (hL * hL) + cL(EN);
+            fd1 = (hR * uR) - (hL * uL);
+            fd2 = phiR - phiL + grav * hbar * (aR[0] - aL[0]);
+        }
         const T fd3 = hR * uR * vR - hL * uL * vL;
         const T s1 = fmin(uL - gL, uhat - chat);
         const T s3 = fmax(uR + gR, uhat + chat);
@@ -450,7 +441,7 @@ struct WaveEulerExact {
         ex[0] = u; ex[1] = v; ex[2] = enth; ex[3] = sqrt(a2); ex[4] = gamma1 / a2;
     }
     template <int IXY, class C>
-    __device__ static int normal(const double* qL, const double* qR, const double*, const double*, C cL, C cR,
+    __device__ static int normal(const double* qL, const double* qR, const double*, const double*, const double*, const double*, C cL, C cR,
                                  const WavePar<double>& P, double seed, State<double>& st, double w[3][4], double* s)
     {
         constexpr int mu = Dir<IXY>::mu, mv = Dir<IXY>::mv;
@@ -562,7 +553,7 @@ struct WaveEulerExact {
     // or u jumps), star states, the Godunov state and the waves in FP32.  FP32 resolves p* to a
     // few ulp, so the iteration stops at a relative change of max(tol, NEWTON_TOL32).
     template <int IXY, class C>
-    __device__ static int normal(const float* qL, const float* qR, const float*, const float*, C cL, C cR,
+    __device__ static int normal(const float* qL, const float* qR, const float*, const float*, const float*, const float*, C cL, C cR,
                                  const WavePar<float>& P, double seed, State<float>& st, float w[3][4], float* s)
     {
         constexpr int mu = Dir<IXY>::mu, mv = Dir<IXY>::mv;
