@@ -92,13 +92,13 @@ def _peaks() -> dict:
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per interior
-# cell-update of the fused update kernel, from one ncu --set full capture of a
+# cell-update of the fused update kernel, from one ncu capture of a
 # 16384-patch launch (radial dam, uniform level 7, 16x16 patches, mbc 2); the
-# summaries are profiles/step2_sw_roe_16x16_<precision>.md.  A launch of n
+# summary is profiles/update_kernels.md.  A launch of n
 # patches moves n * 256 times this.
 DRAM_BYTES_PER_CELL = {
-    ("sw_roe_16x16", "fp32wave"): (158.340352e6 + 89.620224e6) / (16384 * 256),
-    ("sw_roe_16x16", "fp64"): (159.835648e6 + 243.607808e6) / (16384 * 256),
+    ("sw_roe_16x16", "fp32wave"): (158.281472e6 + 92.320768e6) / (16384 * 256),
+    ("sw_roe_16x16", "fp64"): (158.320640e6 + 91.613952e6) / (16384 * 256),
 }
 
 

@@ -3,8 +3,8 @@
     python -m forestclaw_b200.build [--force]
 
 Device code is compiled for sm_100a only.  The FP64 translation units
-(k_step2_f64.cu, k_amr.cu) are compiled with -fmad=false so no FMA contraction
-changes the rounding of the FP64 path; the FP32-wave unit keeps FMA.  Host C++
+(k_step2_f64_*.cu, k_amr.cu) are compiled with -fmad=false so no FMA contraction
+changes the rounding of the FP64 path; the FP32-wave units keep FMA.  Host C++
 is compiled with -ffp-contract=off for the same reason (patch geometry, app
 initial data).  The CUDA runtime is linked statically so the library loads on
 any machine with a driver.

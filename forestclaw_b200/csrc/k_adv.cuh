@@ -25,7 +25,8 @@
 //
 // What bounds it: issue and shared-memory latency (HBM below 15 %); a general kernel that keeps
 // waves, four transverse terms per interface and four flux planes ran at one CTA per SM with
-// six barriers.  Measured: see the table at run_adv_variant.
+// six barriers.  Updates of one coarse step, one B200 (us, ncu, warm): 256 patches of 32x32 FP64
+// 29.3 -> 10.9, cubed sphere levels 3-6, 804 patches of 32x32 FP32-wave 325 -> 131.
 #pragma once
 #include <cuda_runtime.h>
 #include <type_traits>

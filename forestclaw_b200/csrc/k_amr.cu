@@ -393,7 +393,7 @@ struct RegOff {
 // shared memory, prefetched registers and cells there and then computed all corrections before
 // all additions took three barriers and some 240 instructions per item; with the sources in a
 // face-indexed table the chain is source -> neighbour's registers -> add.  Radial dam levels
-// 3-7, 1960 patches: see the figures in launch_sync.
+// 3-7, 16 syncs of 1250 to 1960 patches a step: 192 -> 106 us (6.6 us each).
 // Patch shape and field count of the time sync: compile-time for the common shapes
 // (the index arithmetic and register offsets fold), run-time otherwise.
 template <int MX, int MEQN>

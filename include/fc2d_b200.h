@@ -292,16 +292,18 @@ int fc2d_b200_partition_plan(const fc2d_b200_options_t* opt, int np, const int* 
 /* ---- patch-to-CTA variants of the fused update (no counterpart in the reference) ----
  * Each solver shape (precision, Riemann solver, patch size) is compiled with
  * several mappings of a patch onto its CTA: threads per CTA and an occupancy
- * target (CTAs per SM, which caps registers per thread); reg = 1 when every
+ * target (CTAs per SM, which caps registers per thread), with the method's flags
+ * fixed at compile time where the options match; reg = 1 when every
  * interface of a sweep has its own thread; persistent = 1 for the persistent
- * form (a grid of resident CTAs looping over the level's patches, one launch
- * per level-step however many patches and instances).  Variant 0 is the default.  FP64
- * variants give identical results.  fc2d_b200_autotune times every variant on
+ * form of an application solver (a grid of resident CTAs looping over the level's
+ * patches, one launch per level-step however many patches and instances).  Variant 0 is the
+ * default.  FP64 variants give identical results.  fc2d_b200_autotune times every variant on
  * the current forest (reps passes over all levels, dt = 0 so q is unchanged),
  * keeps the fastest and returns it; ms[v] (may be null, num_variants entries)
- * receives the time of one pass of variant v.  It then times every variant on
- * each level alone and keeps, per level, the fastest there (a level's patch
- * count decides how its CTAs fill the device's waves); fc2d_b200_level_variants
+ * receives the time of one pass of variant v.  A pass is the launches of a coarse step:
+ * a subcycled step updates levels [l, finest] in one launch where they use one variant.
+ * It then times every variant on each level alone and gives a level its own where that
+ * gains more than the launch it splits off; fc2d_b200_level_variants
  * reports the variant each level 0..32 uses.  fc2d_b200_set_variant sets one
  * variant for every level; fc2d_b200_set_level_variants sets each level's (33
  * entries, e.g. another solver's fc2d_b200_level_variants) without timing. */
