@@ -31,6 +31,21 @@ __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 
+// min and max in one instruction that return NaN where an operand is NaN, as the comparisons of
+// dmin1 and dmax1 do below (fminf and fmaxf return the other operand).
+__device__ __forceinline__ float min_nan(float a, float b)
+{
+    float d;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+    float d;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+
 // ---------------------------------------------------------------------------
 // 2D Euler, exact Riemann solver (no counterpart in the reference): the pressure function,
 // fluxes and star pressure.  Newton iteration on p* (Toro, Riemann Solvers and Numerical
@@ -159,7 +174,9 @@ __device__ __forceinline__ T limiter_phi(int mthlim, T r)
     case 3: return (r + fabs(r)) / (T(1) + fabs(r));
     case 4:
         if constexpr (sizeof(T) == 4) {
-            return fmaxf(0.0f, fminf(fminf(fmaf(0.5f, r, 0.5f), 2.0f), 2.0f * r));   // one instruction each
+            // one instruction each.  A ratio of squared waves that overflow FP32 is inf/inf: its NaN
+            // reaches q and the status word, where fminf and fmaxf gave the limiter 2 unnoticed.
+            return max_nan(0.0f, min_nan(min_nan(fmaf(0.5f, r, 0.5f), 2.0f), 2.0f * r));
         } else {
             T c = (T(1) + r) / T(2);
             return dmax1(T(0), dmin1(dmin1(c, T(2)), T(2) * r));
