@@ -45,4 +45,16 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 // for a while in hardware): far beyond any copy of a few KB, short of a hang.
 constexpr int BULK_WAIT_LIMIT = 1 << 20;
 
+// Whether this thread saw the CTA's staging copies (phase 0 of the barrier) arrive.  A translation
+// unit that defines FCB_STAGE_LOST waits all the same but takes them for lost (tests of that path).
+__device__ __forceinline__ bool stage_arrived(unsigned long long* bar)
+{
+    const bool arrived = mbar_wait(bar, 0u, BULK_WAIT_LIMIT);
+#ifdef FCB_STAGE_LOST
+    return false;
+#else
+    return arrived;
+#endif
+}
+
 }  // namespace fcb
