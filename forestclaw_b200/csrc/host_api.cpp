@@ -166,7 +166,7 @@ private:
 
 struct LevelRanges {
     int copy_off = 0, copy_n = 0, avg_off = 0, avg_n = 0, interp_off = 0, interp_n = 0, phys_off = 0, phys_n = 0;
-    int ti_off = 0, ti_n = 0;
+    int ti_off = 0, ti_n = 0, list_off = 0, list_n = 0;
 };
 
 struct fc2d_b200_solver {
@@ -226,6 +226,7 @@ struct fc2d_b200_solver {
     TableArena arena;                              // the tables below, on the device
     DevView<FillOp> t_copy;                        // copy2ghost region ops (cubed sphere)
     DevView<int> t_nbr;                            // copy2ghost neighbours (bricks)
+    DevView<int> t_list;                           // copy2ghost patches of a partitioned brick
     DevView<FillOp> t_avg;                         // average2ghost region ops
     double* area = nullptr;                        // cubed sphere: cell areas per patch (Dims::narea per patch)
     bool sphere = false;                           // the cubed-sphere app (manifold, 6 blocks)
@@ -432,6 +433,8 @@ static int upload_desc_and_tables(fc2d_b200_solver* s)
         if (!build_tables(f, s->o.mthbc, s->has_inflow, T, s->table_work, err)) return fail(FC2D_B200_EFOREST, err);
         s->regrid_ms[4] = wall_ms() - t0;
     }
+    T.copy_list.clear();
+    int list_off[34] = {};
     if (s->part) {
         // partitioned: a new plan for this forest; the ghost-fill stages write only the
         // ghost cells of owned and ring-1 patches, interpolation and the time sync only
@@ -454,8 +457,14 @@ static int upload_desc_and_tables(fc2d_b200_solver* s)
             v.resize(n);
         };
         filter(T.copy, T.copy_off, [&](const FillOp& e) { return fill[e.dst] != 0; });
-        for (size_t k = 0; k < T.copy_nbr.size(); k++)
-            if (!fill[k / 8]) T.copy_nbr[k] = -1;
+        for (int l = 0; l < 33 && !T.copy_nbr.empty(); l++) {
+            list_off[l] = (int)T.copy_list.size();
+            for (int i = f.lev_off[l]; i < f.lev_off[l + 1]; i++) {
+                const int* n = &T.copy_nbr[(size_t)i * 8];
+                if (fill[i] && std::any_of(n, n + 8, [](int v) { return v >= 0; })) T.copy_list.push_back(i);
+            }
+            list_off[l + 1] = (int)T.copy_list.size();
+        }
         filter(T.avg, T.avg_off, [&](const FillOp& e) { return fill[e.dst] != 0; });
         filter(T.phys, T.phys_off, [&](const PhysEnt& e) { return fill[e.dst / nq] != 0; });
         filter(T.interp, T.interp_off, [&](const InterpEnt& e) { return own[e.dst / nq] == me; });
@@ -479,6 +488,7 @@ static int upload_desc_and_tables(fc2d_b200_solver* s)
         r.interp_off = T.interp_off[l]; r.interp_n = T.interp_off[l + 1] - T.interp_off[l];
         r.phys_off = T.phys_off[l]; r.phys_n = T.phys_off[l + 1] - T.phys_off[l];
         r.ti_off = T.ti_off[l]; r.ti_n = T.ti_off[l + 1] - T.ti_off[l];
+        r.list_off = list_off[l]; r.list_n = list_off[l + 1] - list_off[l];
     }
     std::memcpy(s->phys_direct, T.phys_direct, sizeof(s->phys_direct));
     const std::vector<InterpEnt>& interp = T.interp;
@@ -486,11 +496,12 @@ static int upload_desc_and_tables(fc2d_b200_solver* s)
         TableArena& A = s->arena;
         auto sz = [](const auto& v) { return TableArena::span(v.size() * sizeof(v[0])); };
         CK(A.wait_copied());
-        CK(A.reserve(sz(hd) + sz(T.copy) + sz(T.copy_nbr) + sz(T.avg) + sz(T.interp) + sz(T.phys) + sz(T.ti) + sz(T.sync)));
+        CK(A.reserve(sz(hd) + sz(T.copy) + sz(T.copy_nbr) + sz(T.copy_list) + sz(T.avg) + sz(T.interp) + sz(T.phys) + sz(T.ti) + sz(T.sync)));
         A.used = 0;
         const DevView<PatchDesc> dv = A.put(hd);       // staged here, then copied into the slab's descriptors
         s->t_copy = A.put(T.copy);
         s->t_nbr = A.put(T.copy_nbr);
+        s->t_list = A.put(T.copy_list);
         s->t_avg = A.put(T.avg);
         s->t_interp = A.put(T.interp);
         s->t_phys = A.put(T.phys);
@@ -691,6 +702,18 @@ static GatherSeg<E> seg(const E* table, int off, int n, double* dst, const doubl
 {
     return GatherSeg<E>{dst, src, table + off, n};
 }
+// copy2ghost of levels [a, b] of a brick in one array.  A partitioned forest takes the list of the
+// patches this rank fills, so that its launch shrinks with the number of ranks.
+static CopySeg copy_seg(const fc2d_b200_solver* s, double* q, int a, int b)
+{
+    if (s->sphere) return CopySeg{nullptr, 0, 0, nullptr};
+    if (s->part) {
+        const int off = s->lr[a].list_off;
+        return CopySeg{q, 0, s->lr[b].list_off + s->lr[b].list_n - off, s->t_list.p + off};
+    }
+    const int p0 = s->forest.lev_off[a], np = s->forest.lev_off[b + 1] - p0;
+    return CopySeg{q, p0, np > 1 ? np : 0, nullptr};          // a single patch has no neighbours
+}
 // Bytes of the step block's result (status word and CFL maxima).
 static size_t result_bytes(const fc2d_b200_solver* s)
 {
@@ -703,10 +726,8 @@ static size_t result_bytes(const fc2d_b200_solver* s)
 static void average_copy_range(fc2d_b200_solver* s, int a, int b, int ca, int cb, int c, bool phys)
 {
     GatherSeg<PhysEnt> ph{nullptr, nullptr, nullptr, 0};
-
     GatherSeg<FillOp> a0{nullptr, nullptr, nullptr, 0}, a1 = a0, f0 = a0, f1 = a0;
-    CopySeg c0{nullptr, 0, 0}, c1 = c0;
-    const int* lev_off = s->forest.lev_off;
+    CopySeg c0{nullptr, 0, 0, nullptr}, c1 = c0;
     if (lrange(a, b)) {
         const int off = s->lr[a].avg_off, n = s->lr[b].avg_off + s->lr[b].avg_n - off;
         if (n > 0) a0 = seg(s->t_avg.p, off, n, s->q, s->q);
@@ -720,11 +741,11 @@ static void average_copy_range(fc2d_b200_solver* s, int a, int b, int ca, int cb
             const int po = s->lr[ca].phys_off, pn = s->lr[cb].phys_off + s->lr[cb].phys_n - po;
             if (pn > 0) ph = seg(s->t_phys.p, po, pn, s->q, s->q);
         }
-        if (!s->sphere && lev_off[cb + 1] - lev_off[ca] > 1) c0 = CopySeg{s->q, lev_off[ca], lev_off[cb + 1] - lev_off[ca]};
+        c0 = copy_seg(s, s->q, ca, cb);
     }
     if (c >= 0 && c <= 32) {
         if (s->lr[c].copy_n > 0) f1 = seg(s->t_copy.p, s->lr[c].copy_off, s->lr[c].copy_n, s->qinterp, s->qinterp);
-        if (!s->sphere && lev_off[c + 1] - lev_off[c] > 1) c1 = CopySeg{s->qinterp, lev_off[c], lev_off[c + 1] - lev_off[c]};
+        c1 = copy_seg(s, s->qinterp, c, c);
     }
     if (a0.n + a1.n + f0.n + f1.n + c0.np + c1.np + ph.n <= 0) return;
     (void)flush_pending(s);

@@ -166,6 +166,7 @@ void make_partition(const Forest& f, int rank, int size, PartitionPlan& out);
 struct Tables {
     std::vector<FillOp> copy;        // copy2ghost(level) on the cubed sphere: region ops of the level's patches
     std::vector<int> copy_nbr;       // copy2ghost on a brick: 8 same-size neighbours per patch (CopySeg)
+    std::vector<int> copy_list;      // partitioned brick: the patches with such neighbours this rank fills
     std::vector<FillOp> avg;         // average2ghost(level): level is the coarse level
     std::vector<InterpEnt> interp;   // interpolate2ghost(level): level is the coarse level
     std::vector<PhysEnt> phys;       // setphysical(level)

@@ -267,7 +267,9 @@ k_average_copy(GatherSeg<FillOp> a0, GatherSeg<FillOp> a1, GatherSeg<FillOp> f0,
             return;
         }
         const bool second = b >= c0.np;
-        copy_patch(P, second ? c1.q : c0.q, second ? c1.p0 + b - c0.np : c0.p0 + b, nbr, meqn);
+        const int k = second ? b - c0.np : b;
+        const int* list = second ? c1.list : c0.list;
+        copy_patch(P, second ? c1.q : c0.q, list ? list[k] : (second ? c1.p0 : c0.p0) + k, nbr, meqn);
         return;
     }
     const int slot = P.mbc * (P.mx > P.my ? P.mx : P.my);

@@ -82,11 +82,12 @@ struct PhysEnt { int dst, src, neg, cst; };        // neg: bit m set => negate f
 
 // One table segment of a gather stage: entries e[0..n) from src into dst.
 template <class E> struct GatherSeg { double* dst; const double* src; const E* e; int n; };
-// copy2ghost of a brick: patches p0 .. p0 + np - 1 of array q take their ghost cells from their
-// same-size neighbours; nbr[8 p + region] is the neighbour's slot (regions as above), or -1.
+// copy2ghost of a brick: np patches of array q, p0 .. p0 + np - 1 or (list not null, a partitioned
+// forest) list[0 .. np), take their ghost cells from their same-size neighbours;
+// nbr[8 p + region] is the neighbour's slot (regions as above), or -1.
 // Blocks of a brick are equally oriented, so a region's source cells are its own shifted by a
 // patch width.  (The cubed sphere, whose blocks turn, copies by FillOps.)
-struct CopySeg { double* q; int p0, np; };
+struct CopySeg { double* q; int p0, np; const int* list; };
 // average segments and copy segments of one ghost update in one launch (disjoint ghost
 // cells); area: per-patch cell areas (one ring more than q per patch) for the
 // area-weighted average of a manifold, or null for the plain mean.  ph: physical-BC entries that
