@@ -1,6 +1,6 @@
 """A staging copy that does not arrive: the update reports it and writes nothing else.
 
-tests/user_solvers/stage_lost.cu builds the package's kernels so that they take every staging copy
+tests/user_solvers/stage_lost_user.cu builds the package's kernels so that they take every staging copy
 for lost.  q must stay as it was, and so must the values time interpolation starts from
 (save_current_step), which show in the ghost cells it fills; no other failure is reported, although
 the data, were it looked at, holds a negative depth.
@@ -17,7 +17,7 @@ def _module():
     import forestclaw_b200 as fb
     from forestclaw_b200 import build
     fb.load_library()
-    return ctypes.CDLL(next(p for p in build.build_user_examples() if p.endswith("libstage_lost.so")))
+    return ctypes.CDLL(next(p for p in build.build_user_examples() if p.endswith("libstage_lost_user.so")))
 
 
 def _interpolated(g, q):
@@ -29,7 +29,7 @@ def _interpolated(g, q):
     return g.get_q()
 
 
-@pytest.mark.parametrize("how,meqn,maux", [("wave", 3, 0), ("adv", 1, 2)])
+@pytest.mark.parametrize("how,meqn,maux", [("inline", 3, 0), ("advection", 1, 2)])
 def test_lost_staging_copy_writes_nothing(how, meqn, maux):
     import forestclaw_b200 as fb
     g = fb.Solver(fb.Options(mx=8, my=8, mbc=2, meqn=meqn, maux=maux, mwaves=3 if meqn == 3 else 1, minlevel=1, maxlevel=2,
