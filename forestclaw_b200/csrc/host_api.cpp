@@ -2037,9 +2037,9 @@ extern "C" int fc2d_b200_save_step(fc2d_b200_solver_t* s)
     return 0;
 }
 
-extern "C" int fc2d_b200_restore_step(fc2d_b200_solver_t* s)
+// Enqueue the copy back (the run loop retakes its step in stream order, without a wait).
+static int restore_launch(fc2d_b200_solver_t* s)
 {
-    DeviceScope dev_scope_(s);
     if (!s || !s->initialized) return fail(FC2D_B200_ESTATE, "solver not initialized");
     if (s->pending) return fail(FC2D_B200_ESTATE, "an advance is in flight");
     const size_t n = (size_t)s->forest.np() * s->d.nq();
@@ -2049,7 +2049,16 @@ extern "C" int fc2d_b200_restore_step(fc2d_b200_solver_t* s)
     CK(cudaMemcpyAsync(s->q, s->qsave, n * sizeof(double), cudaMemcpyDeviceToDevice, s->st));
     // the ghost cells are back to their saved values, physical ones included
     std::memcpy(s->phys_ok, s->phys_ok_save, sizeof(s->phys_ok));
-    return 0;                                          // in stream order: no wait
+    return 0;
+}
+
+extern "C" int fc2d_b200_restore_step(fc2d_b200_solver_t* s)
+{
+    DeviceScope dev_scope_(s);
+    const int rc = restore_launch(s);
+    if (rc) return rc;
+    CK(cudaStreamSynchronize(s->st));
+    return 0;
 }
 
 // outstyle_1 (src/fclaw2d_run.c:113-265) with reduce_cfl (one process: the global
@@ -2096,7 +2105,7 @@ extern "C" int fc2d_b200_run(fc2d_b200_solver_t* s, fc2d_b200_run_stats_t* out)
                                                    std::to_string(t_curr));
             if (maxcfl_step > o.max_cfl && !o.use_fixed_dt) {
                 // retake the step from the saved copy with a smaller dt
-                if ((rc = fc2d_b200_restore_step(s))) return rc;
+                if ((rc = restore_launch(s))) return rc;
                 if (++retakes > 64) return fail(FC2D_B200_EDEVICE, "fc2d_b200_run: 64 retakes of one step");
                 dt_minlevel = dt_minlevel * o.desired_cfl / maxcfl_step;
                 st.rejected++;

@@ -210,7 +210,8 @@ int fc2d_b200_regrid(fc2d_b200_solver_t* s, int* changed);
 /* patch_vt->save_step / restore_step (fclaw2d_clawpatch.cpp:446-471, called by
  * save_time_step / restore_time_step of src/fclaw2d_run.c:42-82): a device copy of q
  * of every patch (ghosts included), and its return.  The forest must not change
- * in between. */
+ * in between.  save_step enqueues its copy on the solver's stream; restore_step
+ * returns once q is back. */
 int fc2d_b200_save_step(fc2d_b200_solver_t* s);
 int fc2d_b200_restore_step(fc2d_b200_solver_t* s);
 /* fclaw2d_run with outstyle 1 (src/fclaw2d_run.c:113-265) from t = 0 after
