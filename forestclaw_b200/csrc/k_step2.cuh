@@ -33,17 +33,10 @@ namespace fcb {
 
 enum { APP_NONE = 0, APP_SWIRL = 1, APP_RADIALDAM = 2, APP_TSUNAMI = 3, APP_SHOCKBUBBLE = 4 };
 
-// Optional solver hooks.  A solver struct that declares USER_HOOKS = true may also
-// declare HAS_B4STEP2 / HAS_SRC2 with the cell-wise b4step2 / src2 of
-// include/fc2d_b200_user.cuh, and AUX_BOTH = true to receive in rpt2 the aux of
-// both cells beside the interface, cudaclaw's layout (cudaclaw_flux2.cu:682-694):
-// aux1/aux2/aux3[imp * maux + m], imp = 0 for the left cell, 1 for the right.
-template <class RP, class = void>
-struct RPHooks { static constexpr bool B4 = false, SRC = false, AUX_BOTH = false; };
-template <class RP>
-struct RPHooks<RP, std::void_t<decltype(RP::USER_HOOKS)>> {
-    static constexpr bool B4 = RP::HAS_B4STEP2, SRC = RP::HAS_SRC2, AUX_BOTH = RP::AUX_BOTH;
-};
+// A solver struct RP declares HAS_B4STEP2 / HAS_SRC2 with the cell-wise b4step2 / src2 of
+// include/fc2d_b200_user.cuh; its rpt2 receives the aux of both cells beside the interface,
+// cudaclaw's layout (cudaclaw_flux2.cu:682-694): aux1/aux2/aux3[imp * maux + m], imp = 0 for
+// the left cell, 1 for the right.
 
 template <class RP, int MX, int MY, int MBC, typename TW, int NT = 0>
 struct Step2Geom {
@@ -80,7 +73,7 @@ struct Step2Geom {
 
 // The update of patch p by the whole CTA (one call per patch; the CTA may do
 // several patches in turn).
-template <class RP, int MX, int MY, int MBC, bool FWAVE, int NT, typename TW>
+template <class RP, int MX, int MY, int MBC, int NT, typename TW>
 __device__ __forceinline__ void
 step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __restrict__ aux,
             double* __restrict__ regs, const PatchDesc* __restrict__ desc, const int p,
@@ -91,15 +84,9 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     constexpr int NX = G::NX, NY = G::NY, NXY = G::NXY, MEQN = G::MEQN, MWAVES = G::MWAVES;
     constexpr int MAUX = G::MAUX, NEXTRA = G::NEXTRA, NI = G::NI, WSZ = G::WSZ;
     constexpr int MA = MAUX > 0 ? MAUX : 1;
-    // flux2 / flux2fw interface ranges (padded): Godunov, cqxx, amdq+=cqxx, transverse
-    constexpr int GOD_LO = FWAVE ? MBC : 1, GOD_HI = FWAVE ? MX + MBC : NX - 2;
-    constexpr int CQ_LO = FWAVE ? MBC : 1, CQ_HI = FWAVE ? MX + MBC : NX - 1;
-    constexpr int AC_LO = FWAVE ? MBC : 1, AC_HI = FWAVE ? MX + MBC : NX - 2;
-    constexpr int TR_LO = FWAVE ? MBC : 1, TR_HI = FWAVE ? MX + MBC : NX - 1;
-    constexpr int GOD_LOY = FWAVE ? MBC : 1, GOD_HIY = FWAVE ? MY + MBC : NY - 2;
-    constexpr int CQ_LOY = FWAVE ? MBC : 1, CQ_HIY = FWAVE ? MY + MBC : NY - 1;
-    constexpr int AC_LOY = FWAVE ? MBC : 1, AC_HIY = FWAVE ? MY + MBC : NY - 2;
-    constexpr int TR_LOY = FWAVE ? MBC : 1, TR_HIY = FWAVE ? MY + MBC : NY - 1;
+    // flux2 interface ranges (padded): Godunov and amdq+=cqxx up to GOD_HI, cqxx and transverse
+    // at every interface
+    constexpr int GOD_HI = NX - 2, GOD_HIY = NY - 2;
 
     extern __shared__ double smem[];
     double* Qs = smem;                              // [MEQN][NY][NX]
@@ -148,7 +135,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
         }
     }
     __syncthreads();
-    if constexpr (RPHooks<RP>::B4) {
+    if constexpr (RP::HAS_B4STEP2) {
         // user b4step2, cell by cell over the padded patch (cudaclaw_flux2.cu:111-150):
         // it may set the cell's aux from its q, position and time.  As the reference's
         // b4step2 it changes the patch's aux in place (the only write to the aux slab
@@ -211,7 +198,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     // Limiter, second-order correction, fadd and transverse split of one interface.
     // Returns faddm/faddp (FP64) and writes the transverse terms into Tt.
     auto interface_update = [&](int ixy, int k, int cL, int cR, int pos, int lim_lo, int lim_hi,
-                                bool god, bool cqr, bool acr, bool trr, TW dlo, TW dhi, TW dave,
+                                bool god, TW dlo, TW dhi, TW dave,
                                 const int* a1c, const int* a2c, const int* a3c, State& st,
                                 double* faddm, double* faddp) {
         TW cq[MEQN];
@@ -219,8 +206,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
         if (god) {
             for (int m = 0; m < MEQN; m++) { faddp[m] = faddp[m] - (double)st.ap[m]; faddm[m] = faddm[m] + (double)st.am[m]; }
         }
-        const bool second = FWAVE ? (sp.order1 != 1) : (sp.order1 == 2);
-        if (second) {
+        if (sp.order1 == 2) {
             if (pos >= lim_lo && pos <= lim_hi) {
                 // inline limiter (clawpack46_inlinelimiter.f:267-343) with unlimited neighbours;
                 // the neighbours along the sweep are k -+ 1 (x) or k -+ (NX-2) (y)
@@ -243,53 +229,36 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
                     for (int m = 0; m < MEQN; m++) st.wave[mw][m] = wlim * st.wave[mw][m];
                 }
             }
-            if (cqr) {
-                for (int m = 0; m < MEQN; m++) {
-                    TW c = TW(0);
-                    for (int mw = 0; mw < MWAVES; mw++) {
-                        if (FWAVE)
-                            c = add_rn(c, mul_rn(mul_rn(sgn1(st.s[mw]), sub_rn(TW(1), mul_rn(fabs(st.s[mw]), dave))),
-                                                 st.wave[mw][m]));
-                        else {
-                            const TW sa = fabs(st.s[mw]);
-                            c = add_rn(c, mul_rn(mul_rn(sa, sub_rn(TW(1), mul_rn(sa, dave))), st.wave[mw][m]));
-                        }
-                    }
-                    cq[m] = c;
-                    faddm[m] = faddm[m] + (double)(TW(0.5) * c);
-                    faddp[m] = faddp[m] + (double)(TW(0.5) * c);
+            for (int m = 0; m < MEQN; m++) {
+                TW c = TW(0);
+                for (int mw = 0; mw < MWAVES; mw++) {
+                    const TW sa = fabs(st.s[mw]);
+                    c = add_rn(c, mul_rn(mul_rn(sa, sub_rn(TW(1), mul_rn(sa, dave))), st.wave[mw][m]));
                 }
+                cq[m] = c;
+                faddm[m] = faddm[m] + (double)(TW(0.5) * c);
+                faddp[m] = faddp[m] + (double)(TW(0.5) * c);
             }
         }
         unsigned char fl = 0;
-        if (sp.order2 > 0 && trr) {
+        if (sp.order2 > 0) {
             TW am[MEQN], ap[MEQN];
             for (int m = 0; m < MEQN; m++) { am[m] = st.am[m]; ap[m] = st.ap[m]; }
-            if (sp.order1 > 1 && sp.order2 == 2 && acr)
+            if (sp.order1 > 1 && sp.order2 == 2 && god)
                 for (int m = 0; m < MEQN; m++) { am[m] = am[m] + cq[m]; ap[m] = ap[m] - cq[m]; }
             TW qL[MEQN], qR[MEQN];
             for (int m = 0; m < MEQN; m++) { qL[m] = qload(m, cL); qR[m] = qload(m, cR); }
-            constexpr bool BOTH = RPHooks<RP>::AUX_BOTH;
-            TW a1[BOTH ? 2 * MA : MA], a2[BOTH ? 2 * MA : MA], a3[BOTH ? 2 * MA : MA], bm[MEQN], bp[MEQN];
-            if constexpr (BOTH) {
-                for (int h = 0; h < 2; h++)
-                    for (int a = 0; a < MAUX; a++) {
-                        a1[h * MA + a] = (TW)As[a * NXY + a1c[h]];
-                        a2[h * MA + a] = (TW)As[a * NXY + a2c[h]];
-                        a3[h * MA + a] = (TW)As[a * NXY + a3c[h]];
-                    }
-            } else {
-                for (int a = 0; a < MAUX; a++) { a1[a] = (TW)As[a * NXY + a1c[0]]; a2[a] = (TW)As[a * NXY + a2c[0]]; a3[a] = (TW)As[a * NXY + a3c[0]]; }
-            }
+            TW a1[2 * MA], a2[2 * MA], a3[2 * MA], bm[MEQN], bp[MEQN];
+            for (int h = 0; h < 2; h++)
+                for (int a = 0; a < MAUX; a++) {
+                    a1[h * MA + a] = (TW)As[a * NXY + a1c[h]];
+                    a2[h * MA + a] = (TW)As[a * NXY + a2c[h]];
+                    a3[h * MA + a] = (TW)As[a * NXY + a3c[h]];
+                }
             RP::template rpt2<TW>(ixy, 1, qL, qR, a1, a2, a3, st.ex, am, bm, bp, gravw, drytolw);
             for (int m = 0; m < MEQN; m++) {
                 Tt[(0 * MEQN + m) * NI + k] = TW(0.5) * dlo * bm[m];
                 Tt[(1 * MEQN + m) * NI + k] = TW(0.5) * dlo * bp[m];
-            }
-            // (every if-constexpr body here is braced: inside a lambda of a template, nvcc
-            // 12.9 also discards the statement that follows an unbraced discarded `for`)
-            if constexpr (!BOTH) {
-                for (int a = 0; a < MAUX; a++) { a1[a] = (TW)As[a * NXY + a1c[1]]; a2[a] = (TW)As[a * NXY + a2c[1]]; a3[a] = (TW)As[a * NXY + a3c[1]]; }
             }
             RP::template rpt2<TW>(ixy, 2, qL, qR, a1, a2, a3, st.ex, ap, bm, bp, gravw, drytolw);
             for (int m = 0; m < MEQN; m++) {
@@ -311,7 +280,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     auto x2 = [&](int k, State& st) {
         const int jc = 1 + k / (NX - 1), ic = 1 + k % (NX - 1);
         const TW dlo = dtdx1d_x(ic - 1, jc);
-        const TW dhi = FWAVE ? dlo : dtdx1d_x(ic, jc);
+        const TW dhi = dtdx1d_x(ic, jc);
         const TW dave = TW(0.5) * (dtdx1d_x(ic - 1, jc) + dtdx1d_x(ic, jc));
         // aux of cell i1 = ic-1 (amdq) / ic (apdq) on rows jc-1, jc, jc+1
         const int a1c[2] = {(jc - 1) * NX + ic - 1, (jc - 1) * NX + ic};
@@ -319,8 +288,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
         const int a3c[2] = {(jc + 1) * NX + ic - 1, (jc + 1) * NX + ic};
         double faddm[MEQN], faddp[MEQN];
         interface_update(1, k, jc * NX + ic - 1, jc * NX + ic, ic, MBC, MX + MBC,
-                         ic >= GOD_LO && ic <= GOD_HI, ic >= CQ_LO && ic <= CQ_HI, ic >= AC_LO && ic <= AC_HI,
-                         ic >= TR_LO && ic <= TR_HI, dlo, dhi, dave, a1c, a2c, a3c, st, faddm, faddp);
+                         ic <= GOD_HI, dlo, dhi, dave, a1c, a2c, a3c, st, faddm, faddp);
         for (int m = 0; m < MEQN; m++) {
             FMs[m * NXY + jc * NX + ic] = 0.0 + faddm[m];
             FPs[m * NXY + jc * NX + ic] = 0.0 + faddp[m];
@@ -336,7 +304,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     auto y2 = [&](int k, State& st) {
         const int jc = 1 + k / (NX - 2), ic = 1 + k % (NX - 2);
         const TW dlo = dtdy1d_y(ic, jc - 1);
-        const TW dhi = FWAVE ? dlo : dtdy1d_y(ic, jc);
+        const TW dhi = dtdy1d_y(ic, jc);
         const TW dave = TW(0.5) * (dtdy1d_y(ic, jc - 1) + dtdy1d_y(ic, jc));
         // aux of sweep cell i1 = jc-1 (amdq) / jc (apdq) on columns ic-1, ic, ic+1
         const int a1c[2] = {(jc - 1) * NX + ic - 1, jc * NX + ic - 1};
@@ -344,9 +312,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
         const int a3c[2] = {(jc - 1) * NX + ic + 1, jc * NX + ic + 1};
         double faddm[MEQN], faddp[MEQN];
         interface_update(2, k, (jc - 1) * NX + ic, jc * NX + ic, jc, MBC, MY + MBC,
-                         jc >= GOD_LOY && jc <= GOD_HIY, jc >= CQ_LOY && jc <= CQ_HIY,
-                         jc >= AC_LOY && jc <= AC_HIY, jc >= TR_LOY && jc <= TR_HIY, dlo, dhi, dave,
-                         a1c, a2c, a3c, st, faddm, faddp);
+                         jc <= GOD_HIY, dlo, dhi, dave, a1c, a2c, a3c, st, faddm, faddp);
         for (int m = 0; m < MEQN; m++) {
             GMs[m * NXY + jc * NX + ic] = GMs[m * NXY + jc * NX + ic] + faddm[m];
             GPs[m * NXY + jc * NX + ic] = GPs[m * NXY + jc * NX + ic] + faddp[m];
@@ -459,7 +425,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
             qi[m * NXY + c] = add_rn(old, mul_rn(sp.ti_alpha, sub_rn(v, old)));
         }
     };
-    if constexpr (RPHooks<RP>::SRC) {
+    if constexpr (RP::HAS_SRC2) {
         // with a user src2 (clawpack46_update, fc2d_clawpack46.cpp:436-441: src2 after
         // step2), every padded cell gets its updated q (cells the update skips keep
         // theirs) passed through the cell-wise source term before it is stored
@@ -521,7 +487,7 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
 // The fused update of npatch patches starting at slot p0.  One CTA per patch, or
 // (PERSIST) a grid of a few CTAs per SM, each taking patches p0 + blockIdx.x,
 // + gridDim.x, ... in turn, its shared memory reused patch after patch.
-template <class RP, int MX, int MY, int MBC, bool FWAVE, int NT, typename TW, int MINB = 2, bool PERSIST = false>
+template <class RP, int MX, int MY, int MBC, int NT, typename TW, int MINB = 2, bool PERSIST = false>
 __global__ void __launch_bounds__(NT, MINB)
 step2_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __restrict__ aux,
              double* __restrict__ regs, const PatchDesc* __restrict__ desc, int p0, int npatch,
@@ -535,12 +501,12 @@ step2_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* _
         (void)npatch;
         const int p = p0 + (int)blockIdx.x;
         const StepParams sp = spp[group_slot(lg, (int)blockIdx.x)];
-        step2_patch<RP, MX, MY, MBC, FWAVE, NT, TW>(q, qlast, aux, regs, desc, p, sp, cfl_bits);
+        step2_patch<RP, MX, MY, MBC, NT, TW>(q, qlast, aux, regs, desc, p, sp, cfl_bits);
     } else {
         for (int b = blockIdx.x; b < npatch; b += gridDim.x) {
             const int p = p0 + b;
             const StepParams sp = spp[group_slot(lg, b)];
-            step2_patch<RP, MX, MY, MBC, FWAVE, NT, TW>(q, qlast, aux, regs, desc, p, sp, cfl_bits);
+            step2_patch<RP, MX, MY, MBC, NT, TW>(q, qlast, aux, regs, desc, p, sp, cfl_bits);
             __syncthreads();   // the next patch restages the shared memory
         }
     }

@@ -15,7 +15,7 @@
 
 namespace fcb {
 
-template <class RP, int MX, int MBC, bool FW, int NT, int MINB, typename TW, bool PERSIST = false>
+template <class RP, int MX, int MBC, int NT, int MINB, typename TW, bool PERSIST = false>
 cudaError_t run_step2_variant(double* q, double* qlast, const double* aux, double* regs, const PatchDesc* desc,
                               int p0, int npatch, const StepParams* sp, const LevelGroup& lg,
                               unsigned long long* cfl_bits,
@@ -24,7 +24,7 @@ cudaError_t run_step2_variant(double* q, double* qlast, const double* aux, doubl
     using G = Step2Geom<RP, MX, MX, MBC, TW, NT>;
     static bool attr_set = false;
     static int grid_cap = 0;   // persistent: resident CTAs of the whole device
-    auto kern = step2_kernel<RP, MX, MX, MBC, FW, NT, TW, MINB, PERSIST>;
+    auto kern = step2_kernel<RP, MX, MX, MBC, NT, TW, MINB, PERSIST>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM_BYTES);
         if (e != cudaSuccess) return e;
@@ -42,16 +42,5 @@ cudaError_t run_step2_variant(double* q, double* qlast, const double* aux, doubl
     const int grid = PERSIST ? (npatch < grid_cap ? npatch : grid_cap) : npatch;
     return launch_k(kern, grid, NT, G::SMEM_BYTES, st, q, qlast, aux, regs, desc, p0, npatch, sp, lg, cfl_bits);
 }
-
-// One table entry: precision, solver id, square patch size MXV (mbc 2), threads, min CTAs per SM.
-#define FCB_STEP2_VARIANT(PREC, RPID, RPT, MXV, FW, NT, MINB, TW)                                           \
-    Step2Variant{PREC, RPID, MXV, MXV, 2, NT, MINB, Step2Geom<RPT, MXV, MXV, 2, TW, NT>::REG ? 1 : 0,       \
-                 (int)Step2Geom<RPT, MXV, MXV, 2, TW, NT>::SMEM_BYTES, 0,                                   \
-                 &run_step2_variant<RPT, MXV, 2, FW, NT, MINB, TW, false>}
-// The same mapping as a persistent kernel: a grid of resident CTAs looping over the patches.
-#define FCB_STEP2_VARIANT_P(PREC, RPID, RPT, MXV, FW, NT, MINB, TW)                                         \
-    Step2Variant{PREC, RPID, MXV, MXV, 2, NT, MINB, Step2Geom<RPT, MXV, MXV, 2, TW, NT>::REG ? 1 : 0,       \
-                 (int)Step2Geom<RPT, MXV, MXV, 2, TW, NT>::SMEM_BYTES, 1,                                   \
-                 &run_step2_variant<RPT, MXV, 2, FW, NT, MINB, TW, true>}
 
 }  // namespace fcb

@@ -76,7 +76,6 @@ constexpr int user_threads() { return MX <= 8 ? 128 : (MX <= 16 ? 352 : 512); }
 template <int MEQN_, int MWAVES_, int MAUX_, class Impl>
 struct RPUserBase {
     static constexpr int MEQN = MEQN_, MWAVES = MWAVES_, MAUX = MAUX_, NEXTRA = 1;
-    static constexpr bool USER_HOOKS = true, AUX_BOTH = true;
     static constexpr int MA = MAUX > 0 ? MAUX : 1;
     template <typename T>
     __device__ static void rpn2(int ixy, const T* qL, const T* qR, const T* auxL, const T* auxR,
@@ -150,7 +149,7 @@ struct RPUserPtr : RPUserBase<MEQN_, MWAVES_, MAUX_, RPUserPtr<MEQN_, MWAVES_, M
                       fcb::Step2Geom<RPT, MXV, MXV, 2, double, fcb::user_threads<MXV>()>::REG ? 1 : 0,        \
                       (int)fcb::Step2Geom<RPT, MXV, MXV, 2, double, fcb::user_threads<MXV>()>::SMEM_BYTES,     \
                       PERSIST,                                                                               \
-                      &fcb::run_step2_variant<RPT, MXV, 2, false, fcb::user_threads<MXV>(), (MXV > 16 ? 1 : 2), \
+                      &fcb::run_step2_variant<RPT, MXV, 2, fcb::user_threads<MXV>(), (MXV > 16 ? 1 : 2), \
                                               double, PERSIST>}
 #define FC2D_B200_USER_TABLE_(RPT, MXV) FC2D_B200_USER_VARIANT_(RPT, MXV, 0), FC2D_B200_USER_VARIANT_(RPT, MXV, 1)
 
