@@ -91,14 +91,15 @@ def _peaks() -> dict:
     return {"hbm_gbs": 6650.0, "source": "fallback"}
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per interior
-# cell-update of the fused update kernel, from one ncu capture of a
-# 16384-patch launch (radial dam, uniform level 7, 16x16 patches, mbc 2); the
-# summary is profiles/update_kernels.md.  A launch of n
-# patches moves n * 256 times this.
+# DRAM bytes per interior cell-update of the fused update kernel, radial dam, 16x16
+# patches, mbc 2: read, dram__bytes_read.sum of one 16384-patch launch (uniform level
+# 7); written, the 19x19 cells of 3 FP64 fields the kernel stores per patch (that
+# launch's dram__bytes_write.sum, 92 MB of 142, leaves out what is still in L2).  A
+# launch of n patches moves n * 256 times this.
+_STORED_PER_PATCH = 19 * 19 * 3 * 8
 DRAM_BYTES_PER_CELL = {
-    ("sw_roe_16x16", "fp32wave"): (158.281472e6 + 92.320768e6) / (16384 * 256),
-    ("sw_roe_16x16", "fp64"): (158.320640e6 + 91.613952e6) / (16384 * 256),
+    ("sw_roe_16x16", "fp32wave"): (158.254848e6 / 16384 + _STORED_PER_PATCH) / 256,
+    ("sw_roe_16x16", "fp64"): (158.274560e6 / 16384 + _STORED_PER_PATCH) / 256,
 }
 
 

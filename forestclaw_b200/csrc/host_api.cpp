@@ -559,7 +559,8 @@ static StepParams make_params(const fc2d_b200_solver* s, int level, double t, do
     sp.mcapa = s->o.mcapa;
     sp.store_flux = s->o.time_sync && s->o.flux_correction;
     sp.accumulate_waves = s->o.time_sync && s->o.fluctuation_correction;
-    // save_current_step is only read by time interpolation of the coarser levels
+    // save_current_step is only read by k_timeinterp, of the coarser levels: on a partitioned forest
+    // and in the C entry (an advance of one rank interpolates in the update)
     sp.save_last = (s->o.subcycle && level < f.maxlevel_present) ? 1 : 0;
     sp.app = s->o.app;
     // reflecting walls whose ghost cells mirror the interior (FP32-wave mass rule)

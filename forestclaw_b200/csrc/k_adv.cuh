@@ -226,8 +226,8 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
 
     // ---- cells -------------------------------------------------------------------
     unsigned bad = 0;        // STATUS_* found in this thread's cells
-    // save_current_step: only the data time interpolation will read (coarser
-    // levels of a subcycled step, patches with fine-grid neighbours)
+    // save_current_step: only what k_timeinterp may read (coarser levels of a subcycled step, patches
+    // with fine-grid neighbours); an advance of one rank interpolates below instead
     const bool save = arrived && sp->save_last && (pd->flags & PATCH_HAS_FINE_NBR);
     // b4step2: aux(:,:,1) = vty*(psi(x,y+dy)-psi), aux(:,:,2) = -vtx*(psi(x+dx,y)-psi); the
     // stored aux holds the psi differences

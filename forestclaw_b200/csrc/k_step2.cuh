@@ -106,8 +106,8 @@ step2_patch(double* __restrict__ q, double* __restrict__ qlast, const double* __
     const double dt = sp.inst_dt ? sp.dt * sp.inst_dt[pd.inst] : sp.dt;
     const double dtdx = dt / dx, dtdy = dt / dy;
     double* qg = q + (size_t)p * MEQN * NXY;
-    // save_current_step: only the data time interpolation will read (coarser
-    // levels of a subcycled step, patches with fine-grid neighbours)
+    // save_current_step: only what k_timeinterp may read (coarser levels of a subcycled step, patches
+    // with fine-grid neighbours); an advance of one rank interpolates below instead
     const bool save = sp.save_last && (pd.flags & PATCH_HAS_FINE_NBR);
 
     // ---- stage q (and aux) in shared memory --------------------------------

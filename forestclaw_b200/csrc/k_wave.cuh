@@ -24,7 +24,8 @@
 // reproduce that cancellation only to FP32 rounding (about 1e-8 of the mass per step), so the
 // FP32-wave form takes the exact value, zero, for the mass component there.
 //
-// What bounds it: instruction issue and, at 11 warps per CTA, latency; HBM is below 10 %.  So
+// What bounds it: instruction issue (54 to 72 % of the slots in the shallow-water forms, 36 to 53 %
+// in Euler's) and, at 11 or 12 warps per CTA and one to three CTAs per SM, latency; HBM is below 11 %.  So
 // what counts is instructions per interface and CTAs per SM.  Against a kernel that solved
 // each interface from the bare states and kept four flux planes per cell:
 //   * square roots, sound speeds and velocities are formed once per cell for both sweeps
@@ -32,7 +33,8 @@
 //     fluxes, which are first written after their last use;
 //   * fluxes are stored per interface, not per cell, and nothing is zeroed;
 //   * an interface keeps only what its second phase cannot form again, so two FP64 CTAs of
-//     a 16x16 shallow-water patch fit an SM without spills;
+//     a 16x16 shallow-water patch fit an SM (80 registers; spill stores of the variant used by
+//     default: Roe 8 bytes, f-wave 40);
 //   * the limiter reads the upwind neighbour's wave only;
 //   * LIM > 0 fixes the method at compile time (second order, second-order transverse terms,
 //     that limiter on every wave); LIM = 0 reads it from the launch's parameters.
@@ -441,8 +443,8 @@ wave_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __
 
     // ---- cells -------------------------------------------------------------------
     unsigned bad = 0;        // STATUS_* found in this thread's cells
-    // save_current_step: only the data time interpolation will read (coarser
-    // levels of a subcycled step, patches with fine-grid neighbours)
+    // save_current_step: only what k_timeinterp may read (coarser levels of a subcycled step, patches
+    // with fine-grid neighbours); an advance of one rank interpolates below instead
     const bool save = arrived && sp->save_last && (pd->flags & PATCH_HAS_FINE_NBR);
     for (int c = tid; c < NXY; c += NT) {
         double qv[MEQN];
