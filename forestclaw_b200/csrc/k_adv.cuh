@@ -219,16 +219,17 @@ adv_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __r
     const int bcc = (pd->flags / PATCH_BCC3) & 15;
     const AdvPatch<RP, MX, TW, LIM> X{sm, AdvMethod<LIM, RP::CAPA>(sp), dt / dx, dt / dy, dx == dy};
     double* Q = X.Q();
+    // save_current_step: only what k_timeinterp may read (coarser levels of a subcycled step, patches
+    // with fine-grid neighbours); an advance of one rank interpolates below instead
+    bool save = sp->save_last && (pd->flags & PATCH_HAS_FINE_NBR);      // read while the copies travel
     __syncthreads();                                        // the barrier word is initialised
     // a thread that does not see the copies arrive writes nothing but the report of it (a decision
     // of the whole CTA before the cells phase, by thread 0 alone, took 0.8 % longer)
     const bool arrived = stage_arrived(bar);
+    save = save && arrived;
 
     // ---- cells -------------------------------------------------------------------
     unsigned bad = 0;        // STATUS_* found in this thread's cells
-    // save_current_step: only what k_timeinterp may read (coarser levels of a subcycled step, patches
-    // with fine-grid neighbours); an advance of one rank interpolates below instead
-    const bool save = arrived && sp->save_last && (pd->flags & PATCH_HAS_FINE_NBR);
     // b4step2: aux(:,:,1) = vty*(psi(x,y+dy)-psi), aux(:,:,2) = -vtx*(psi(x+dx,y)-psi); the
     // stored aux holds the psi differences
     const bool swirl = sp->app == FC2D_B200_APP_SWIRL;

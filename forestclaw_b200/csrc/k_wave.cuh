@@ -436,16 +436,17 @@ wave_kernel(double* __restrict__ q, double* __restrict__ qlast, const double* __
     WP X{sm, WaveMethod<LIM>(sp), WavePar<TW>{(TW)sp->grav, (TW)sp->dry_tolerance, sp->gamma, sp->newton_tol, konst},
          sp->grav, dt / dx, dt / dy, wallf};
     double* Q = X.Q();
+    // save_current_step: only what k_timeinterp may read (coarser levels of a subcycled step, patches
+    // with fine-grid neighbours); an advance of one rank interpolates below instead
+    bool save = sp->save_last && (pd->flags & PATCH_HAS_FINE_NBR);      // read while the copies travel
     __syncthreads();                                        // the barrier word is initialised
     // a thread that does not see the copies arrive writes nothing but the report of it (a decision
     // of the whole CTA before the cells phase, by thread 0 alone, took 0.8 % longer)
     const bool arrived = stage_arrived(bar);
+    save = save && arrived;
 
     // ---- cells -------------------------------------------------------------------
     unsigned bad = 0;        // STATUS_* found in this thread's cells
-    // save_current_step: only what k_timeinterp may read (coarser levels of a subcycled step, patches
-    // with fine-grid neighbours); an advance of one rank interpolates below instead
-    const bool save = arrived && sp->save_last && (pd->flags & PATCH_HAS_FINE_NBR);
     for (int c = tid; c < NXY; c += NT) {
         double qv[MEQN];
         TW qt[MEQN], cv[RP::NPRE];
